@@ -57,6 +57,60 @@ template <class R> __device__ __forceinline__ R pfloor(R f, R p0) {
   if constexpr (PDev<R>::on) return f - p0; else return f;
 }
 
+// ------------------------------------------------------------------ shared denominators
+// q[n] = x[n] / b for n < N, each the correctly rounded quotient, from one reciprocal.
+// With r = 1 / b correctly rounded, two residual steps take x * r to the rounded quotient
+// (Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor",
+// IBM J. Res. Dev. 34, 1990: the first step gives a quotient within one unit in the last
+// place, and from such a quotient and the rounded reciprocal the second gives the rounded
+// one), as long as nothing under- or overflows. That holds for b and x within
+// 2^-500..2^500; x = 0 gives the signed zero. If any operand of the group lies outside
+// (subnormal, infinite or NaN ones among them), the whole group is divided plainly.
+// Why: the mixture states divide every species by the same density, and N plain divisions
+// are N reciprocals, each with its own branch to the special cases, which keep the
+// compiler from overlapping them; here the N chains are independent straight-line code.
+__device__ __forceinline__ bool quot_plain(double x) {
+  const int h = __double2hiint(x) & 0x7fffffff;
+  return unsigned(h - 0x20b00000) < 0x3e900000u || (h | __double2loint(x)) == 0;
+}
+template <int N>
+__device__ __forceinline__ void div_all(const double* x, double b, double r, double* q) {
+  bool ok = unsigned((__double2hiint(b) & 0x7fffffff) - 0x20b00000) < 0x3e900000u;
+#pragma unroll
+  for (int n = 0; n < N; ++n) ok = ok && quot_plain(x[n]);
+  // the operands are checked first, so that a quotient can take its numerator's registers
+  if (ok) {
+    const int sb = __double2hiint(b);
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+      const int sign = (__double2hiint(x[n]) ^ sb) & 0x80000000;
+      const double q0 = x[n] * r;
+      const double q1 = fma(fma(-b, q0, x[n]), r, q0);
+      const double q2 = fma(fma(-b, q1, x[n]), r, q1);
+      // the sign from the operands: the residual steps lose the sign of a zero
+      q[n] = __hiloint2double((__double2hiint(q2) & 0x7fffffff) | sign, __double2loint(q2));
+    }
+  } else {
+#pragma unroll
+    for (int n = 0; n < N; ++n) q[n] = x[n] / b;
+  }
+}
+template <int N>
+__device__ __forceinline__ void div_all(const double* x, double b, double* q) {
+  if constexpr (N < 6) {
+    // a group this small gains nothing from the shared reciprocal (one-species states)
+#pragma unroll
+    for (int n = 0; n < N; ++n) q[n] = x[n] / b;
+  } else {
+    div_all<N>(x, b, 1.0 / b, q);
+  }
+}
+template <int N>
+__device__ __forceinline__ void div_all(const float* x, float b, float* q) {
+#pragma unroll
+  for (int n = 0; n < N; ++n) q[n] = x[n] / b;
+}
+
 // ------------------------------------------------------------------ views
 // Element offsets within one view are 32-bit: the host refuses arrays whose component
 // extent (ncomp * nstride) or strides reach 2^31 elements (pcg::kMaxViewElems), so every
@@ -779,8 +833,10 @@ __device__ __forceinline__ void riemann(const FaceState<NS, R>& L, const FaceSta
   const R cr = E::rpy2cs(rr, pr, Rs.y);
   const R wl = dmax(wsmall, cl * rl);
   const R wr = dmax(wsmall, cr * rr);
-  const R pstar = dmax(Lim<R>::tiny(), ((wr * pl + wl * pr) + wl * wr * (ul - ur)) / (wl + wr));
-  R ustar = ((wl * ul + wr * ur) + (pl - pr)) / (wl + wr);
+  R star[2] = {(wr * pl + wl * pr) + wl * wr * (ul - ur), (wl * ul + wr * ur) + (pl - pr)};
+  div_all<2>(star, wl + wr, star);
+  const R pstar = dmax(Lim<R>::tiny(), star[0]);
+  R ustar = star[1];
 
   bool mask = ustar > R(0);
   R rspo[NS];
@@ -804,8 +860,7 @@ __device__ __forceinline__ void riemann(const FaceState<NS, R>& L, const FaceSta
   po = mask ? R(0.5) * (pl + pr) : po;
 
   R ytmp[NS];
-#pragma unroll
-  for (int n = 0; n < NS; n++) ytmp[n] = rspo[n] / ro;
+  div_all<NS>(rspo, ro, ytmp);
   const R co = E::rpy2cs(ro, po, ytmp);
 
   const R drho = (pstar - po) / (co * co);
@@ -813,12 +868,10 @@ __device__ __forceinline__ void riemann(const FaceState<NS, R>& L, const FaceSta
   R rstar = R(0);
 #pragma unroll
   for (int n = 0; n < NS; n++) {
-    const R spon = rspo[n] / ro;
-    rspstar[n] = dmax(R(0), rspo[n] + drho * spon);
+    rspstar[n] = dmax(R(0), rspo[n] + drho * ytmp[n]);
     rstar += rspstar[n];
   }
-#pragma unroll
-  for (int n = 0; n < NS; n++) ytmp[n] = rspstar[n] / rstar;
+  div_all<NS>(rspstar, rstar, ytmp);
   const R cstar = E::rpy2cs(rstar, pstar, ytmp);
 
   const R sgnm = copysign(R(1), ustar);
@@ -858,8 +911,7 @@ __device__ __forceinline__ void riemann(const FaceState<NS, R>& L, const FaceSta
   qint_iu = mask ? ustar : qint_iu;
   qint_gdpres = mask ? pstar : qint_gdpres;
 
-#pragma unroll
-  for (int n = 0; n < NS; n++) ytmp[n] = rspgd[n] / rgd;
+  div_all<NS>(rspgd, rgd, ytmp);
   const R gdnv_e = E::ryp2e(rgd, ytmp, qint_gdpres);
   const R regd = rgd * gdnv_e;
 

@@ -165,11 +165,11 @@ __global__ void __launch_bounds__(128, MINB) k_ctoprim(pcg::StageArgs a) {
   const double kineng = 0.5 * rho * (vx * vx + vy * vy + vz * vz) - 0.5 * rho * 0.0 * 0.0 * 0.0 * 0.0;
   double y[NS];
 #pragma unroll
-  for (int n = 0; n < NS; n++) {
-    double yn = u[pcg::UFS + n] / rho;
-    if ((-1e-4 * DBL_EPSILON < yn) && (yn < 1e-4 * DBL_EPSILON)) yn = 0.0;
-    y[n] = yn;
-  }
+  for (int n = 0; n < NS; n++) y[n] = u[pcg::UFS + n];
+  div_all<NS>(y, rho, rhoinv, y);
+#pragma unroll
+  for (int n = 0; n < NS; n++)
+    if ((-1e-4 * DBL_EPSILON < y[n]) && (y[n] < 1e-4 * DBL_EPSILON)) y[n] = 0.0;
   const double e = (u[pcg::UEDEN] - kineng) * rhoinv;
   const double wbar = E::y2wbar(y);
   const double T = E::rey2t(e, y, u[pcg::UTEMP]);
@@ -990,6 +990,7 @@ __device__ __forceinline__ void transdo_apply(const R* qn, const KF& K, R p0, R*
   const R rr = qn[pcg::TR_RHO];
   const R rrnew = rr - flxrho;
   const R irrnew = EXACT ? R(0) : rrcp(rrnew);
+  R num[NS + 4];  // EXACT: the numerators over rrnew, divided together
   if constexpr (sizeof(R) == 4 && NS > 1) {
     R kc[NS];
 #pragma unroll
@@ -999,8 +1000,8 @@ __device__ __forceinline__ void transdo_apply(const R* qn, const KF& K, R p0, R*
 #pragma unroll
     for (int n = 0; n < NS; n++) {
       const R compn = K(pcg::FL_Y + n);
-      const R compo = rr * qn[pcg::TR_Y + n] - compn;
-      out[pcg::TR_Y + n] = EXACT ? compo / rrnew : compo * irrnew;
+      num[n] = rr * qn[pcg::TR_Y + n] - compn;
+      if (!EXACT) out[pcg::TR_Y + n] = num[n] * irrnew;
     }
   }
   R ru = qn[pcg::TR_U], rv = qn[pcg::TR_V], rw = qn[pcg::TR_W];
@@ -1013,12 +1014,21 @@ __device__ __forceinline__ void transdo_apply(const R* qn, const KF& K, R p0, R*
   const R rvnew = rv - flxv;
   const R rwnew = rw - flxw;
   const R renew = re - flxe;
-  out[pcg::TR_RHO] = rrnew;
-  out[pcg::TR_U] = EXACT ? runew / rrnew : runew * irrnew;
-  out[pcg::TR_V] = EXACT ? rvnew / rrnew : rvnew * irrnew;
-  out[pcg::TR_W] = EXACT ? rwnew / rrnew : rwnew * irrnew;
   const R ke2 = runew * runew + rvnew * rvnew + rwnew * rwnew;
-  const R rhoekin = EXACT ? R(0.5) * ke2 / rrnew : R(0.5) * ke2 * irrnew;
+  if constexpr (EXACT) {
+    num[NS] = runew;
+    num[NS + 1] = rvnew;
+    num[NS + 2] = rwnew;
+    num[NS + 3] = R(0.5) * ke2;
+    div_all<NS + 4>(num, rrnew, num);
+#pragma unroll
+    for (int n = 0; n < NS; n++) out[pcg::TR_Y + n] = num[n];
+  }
+  out[pcg::TR_RHO] = rrnew;
+  out[pcg::TR_U] = EXACT ? num[NS] : runew * irrnew;
+  out[pcg::TR_V] = EXACT ? num[NS + 1] : rvnew * irrnew;
+  out[pcg::TR_W] = EXACT ? num[NS + 2] : rwnew * irrnew;
+  const R rhoekin = EXACT ? num[NS + 3] : R(0.5) * ke2 * irrnew;
   out[pcg::TR_RE] = renew - rhoekin;
   const R pnew = qn[pcg::TR_P] - K(5 + NS);
   out[pcg::TR_P] = dmax(pnew, pfloor(Lim<R>::very_small(), p0));
@@ -1285,6 +1295,7 @@ __device__ __forceinline__ void transdd_apply(const R* qn, const R* K, R hdt, bo
   const R rr = qn[pcg::TR_RHO];
   const R rrnew = rr - flxrho;
   const R irrnew = EXACT ? R(0) : rrcp(rrnew);
+  R num[NS + 4];  // EXACT: the numerators over rrnew, divided together
   if constexpr (sizeof(R) == 4 && NS > 1) {
     scale_sub2<NS>(rr, qn + pcg::TR_Y, K + pcg::FL_Y, irrnew, out + pcg::TR_Y);
     if (has_src) {
@@ -1294,10 +1305,9 @@ __device__ __forceinline__ void transdd_apply(const R* qn, const R* K, R hdt, bo
   } else {
 #pragma unroll
     for (int n = 0; n < NS; n++) {
-      const R srcpass = has_src ? R(sq[pcg::QFS + n]) : R(0);
       const R compn = K[pcg::FL_Y + n];
-      const R compo = rr * qn[pcg::TR_Y + n] - compn;
-      out[pcg::TR_Y + n] = (EXACT ? compo / rrnew : compo * irrnew) + hdt * srcpass;
+      num[n] = rr * qn[pcg::TR_Y + n] - compn;
+      if (!EXACT) out[pcg::TR_Y + n] = num[n] * irrnew + hdt * (has_src ? R(sq[pcg::QFS + n]) : R(0));
     }
   }
   const R pxnew = K[5 + NS];
@@ -1315,12 +1325,21 @@ __device__ __forceinline__ void transdd_apply(const R* qn, const R* K, R hdt, bo
   const R rvnew = rv - flxv;
   const R rwnew = rw - flxw;
   const R renew = re - flxe;
-  out[pcg::TR_RHO] = rrnew + hdt * s0;
-  out[pcg::TR_U] = (EXACT ? runew / rrnew : runew * irrnew) + hdt * s1;
-  out[pcg::TR_V] = (EXACT ? rvnew / rrnew : rvnew * irrnew) + hdt * s2;
-  out[pcg::TR_W] = (EXACT ? rwnew / rrnew : rwnew * irrnew) + hdt * s3;
   const R ke2 = runew * runew + rvnew * rvnew + rwnew * rwnew;
-  const R rhoekin = EXACT ? R(0.5) * ke2 / rrnew : R(0.5) * ke2 * irrnew;
+  if constexpr (EXACT) {
+    num[NS] = runew;
+    num[NS + 1] = rvnew;
+    num[NS + 2] = rwnew;
+    num[NS + 3] = R(0.5) * ke2;
+    div_all<NS + 4>(num, rrnew, num);
+#pragma unroll
+    for (int n = 0; n < NS; n++) out[pcg::TR_Y + n] = num[n] + hdt * (has_src ? R(sq[pcg::QFS + n]) : R(0));
+  }
+  out[pcg::TR_RHO] = rrnew + hdt * s0;
+  out[pcg::TR_U] = (EXACT ? num[NS] : runew * irrnew) + hdt * s1;
+  out[pcg::TR_V] = (EXACT ? num[NS + 1] : rvnew * irrnew) + hdt * s2;
+  out[pcg::TR_W] = (EXACT ? num[NS + 2] : rwnew * irrnew) + hdt * s3;
+  const R rhoekin = EXACT ? num[NS + 3] : R(0.5) * ke2 * irrnew;
   out[pcg::TR_RE] = renew - rhoekin + hdt * s4;
   const R pn = qn[pcg::TR_P] - pxnew - pynew + hdt * s5;
   out[pcg::TR_P] = dmax(pn, pfloor(Lim<R>::tiny(), p0));
@@ -1733,19 +1752,22 @@ __device__ __forceinline__ void consup_each(const pcg::Region& rg, int i, int j,
   const double a1m = ua ? a1(i, j, k) : rg.area_u[1], a1p = ua ? a1(i, j + 1, k) : rg.area_u[1];
   const double a2m = ua ? a2(i, j, k) : rg.area_u[2], a2p = ua ? a2(i, j, k + 1) : rg.area_u[2];
   const double v = rg.vol.p ? v4<const double>(rg.vol)(i, j, k) : rg.vol_u;
-  const double pdivu = 0.5 *
-                       ((double(q0p[0]) + p0 + (double(q0[0]) + p0)) * (double(q0p[1]) * a0p - double(q0[1]) * a0m) +
-                        (double(q1p[0]) + p0 + (double(q1[0]) + p0)) * (double(q1p[1]) * a1p - double(q1[1]) * a1m) +
-                        (double(q2p[0]) + p0 + (double(q2[0]) + p0)) * (double(q2p[1]) * a2p - double(q2[1]) * a2m)) /
-                       v;
+  // the volume divides every component's flux sum and the p div u term: divided together
+  constexpr int NV = pcg::nvar(NS);
+  double num[NV + 1];
+#pragma unroll
+  for (int n = 0; n < NV; ++n)
+    num[n] = double(f0[n]) - double(f0p[n]) + double(f1[n]) - double(f1p[n]) + double(f2[n]) - double(f2p[n]);
+  num[NV] = 0.5 * ((double(q0p[0]) + p0 + (double(q0[0]) + p0)) * (double(q0p[1]) * a0p - double(q0[1]) * a0m) +
+                   (double(q1p[0]) + p0 + (double(q1[0]) + p0)) * (double(q1p[1]) * a1p - double(q1[1]) * a1m) +
+                   (double(q2p[0]) + p0 + (double(q2[0]) + p0)) * (double(q2p[1]) * a2p - double(q2[1]) * a2m));
+  div_all<NV + 1>(num, v, num);
   const CellPtr<double> uo = at(v4<double>(rg.uout), i, j, k);
 #pragma unroll
-  for (int n = 0; n < pcg::nvar(NS); ++n) {
+  for (int n = 0; n < NV; ++n) {
     const double old = rg.zero_uout ? 0.0 : uo[n];
-    double h = old + (double(f0[n]) - double(f0p[n]) + double(f1[n]) - double(f1p[n]) + double(f2[n]) -
-                      double(f2p[n])) /
-                         v;
-    if (n == pcg::UEINT) h -= pdivu;
+    double h = old + num[n];
+    if (n == pcg::UEINT) h -= num[NV];
     out(n, h);
   }
 }
