@@ -169,6 +169,8 @@ template <bool MIX> struct EosC<double, MIX> {
   static __device__ __forceinline__ double cvr(int k, int r, int i) { return e().cvc[k][r][i]; }
   static __device__ __forceinline__ double ecr(int k, int r, int i) { return e().ec[k][r][i]; }
   static __device__ __forceinline__ double gamma() { return e().gamma; }
+  static __device__ __forceinline__ double star_lo() { return e().star_lo; }
+  static __device__ __forceinline__ double star_hi() { return e().star_hi; }
   static __device__ __forceinline__ double imw(int k) { return e().imw[k]; }
   static __device__ __forceinline__ double tmid(int k) { return e().tmid[k]; }
   static __device__ __forceinline__ const double* cv(int k, int r) { return e().cvc[k][r]; }
@@ -180,6 +182,8 @@ template <bool MIX> struct EosC<float, MIX> {
   static __device__ __forceinline__ float cvr(int k, int r, int i) { return e().cvcf[k][r][i]; }
   static __device__ __forceinline__ float ecr(int k, int r, int i) { return e().ecf[k][r][i]; }
   static __device__ __forceinline__ float gamma() { return e().gammaf; }
+  static __device__ __forceinline__ float star_lo() { return e().star_lof; }
+  static __device__ __forceinline__ float star_hi() { return e().star_hif; }
   static __device__ __forceinline__ float imw(int k) { return e().imwf[k]; }
   static __device__ __forceinline__ float tmid(int k) { return e().tmidf[k]; }
   static __device__ __forceinline__ const float* cv(int k, int r) { return e().cvcf[k][r]; }
@@ -716,15 +720,30 @@ struct RiemannOut {
   R gut1, gut2, regd;  // the Godunov state's tangential velocities and rho*e (qint)
 };
 
+// Whether the star state is the Godunov state beyond doubt: the two-shock solver takes it
+// where spin >= 0, with spin = cstar - |ustar| in a rarefaction and the mean of that and
+// spout in a shock. cstar^2 = (1 + rmix / cv) pstar / rstar exceeds pstar / rstar wherever cv
+// is positive, so ustar^2 rstar <= 0.98 pstar (1 % of margin in the speed, far above
+// rounding) decides it without cstar, its EOS evaluation and the fan blend. cv is positive
+// in the table's temperature range EosConst::star_lo/hi; the bounds on pstar / rstar
+// keep T in it for any composition. Every comparison fails for NaN, which leaves the
+// decision to the full expressions. Subsonic flow decides nearly every face here.
+template <bool MIX, class R>
+__device__ __forceinline__ bool star_certain(R pstar, R rstar, R ustar, bool rarefaction, R spout) {
+  return ustar * ustar * rstar <= R(0.98) * pstar && EosC<R, MIX>::star_lo() * rstar <= pstar &&
+         pstar <= EosC<R, MIX>::star_hi() * rstar && (rarefaction || spout >= R(0));
+}
+
 // Source/Riemann.H:9-200 (riemann), omega = rad = 0, bc_test_val = 1. The EOS calls
 // whose results the reference overwrites unused (RYP2E at :94, :111, :153) are not
 // evaluated; they do not affect any output.
 // Source/Riemann.H:9-200 in the reduced algebra of the FMA/mixed forms (see EosR):
 // the same states, masks and blends, with the species normalisations folded into one
 // reciprocal per state and rho*e of the Godunov state taken directly as
-// sum(rho Y_k e_k(T)).
-template <int NS, bool MIX, class R>
-__device__ __forceinline__ void riemann_reduced(const FaceState<NS, R>& L, const FaceState<NS, R>& Rs, R cav,
+// sum(rho Y_k e_k(T)). cav() is the mean sound speed of the two cells, which only a fan of
+// zero width reads.
+template <int NS, bool MIX, class R, class CAV>
+__device__ __forceinline__ void riemann_reduced(const FaceState<NS, R>& L, const FaceState<NS, R>& Rs, const CAV& cav,
                                                 R p0, RiemannOut<R>& o) {
   using ER = EosR<NS, MIX, R>;
   const R rl = L.rho, ul = L.un, vl = L.ut1, v2l = L.ut2, pl = L.p;
@@ -772,36 +791,47 @@ __device__ __forceinline__ void riemann_reduced(const FaceState<NS, R>& L, const
     rspstar[n] = dmax(R(0), rspo[n] * gscale);
     rstar += rspstar[n];
   }
-  const R cstar = ER::cs_w(rstar, pabs(pstar, p0), rspstar);
-  const R sgnm = copysign(R(1), ustar);
-  R spout = co - sgnm * uo;
-  R spin = cstar - sgnm * ustar;
-  const R ushock = R(0.5) * (spin + spout);
-  mask = pstar < po;
-  spout = mask ? spout : ushock;
-  spin = mask ? spin : ushock;
-  const R scr = (fabs(spout - spin) < Lim<R>::very_small()) ? R(pcg::SMALL_NUM) * cav : spout - spin;
-  const R frac = max0_min1<R>((R(1) + rdiv(spout + spin, scr)) * R(0.5));
   mask = ustar > R(0);
   R qint_iv1 = mask ? vl : vr;
   R qint_iv2 = mask ? v2l : v2r;
   mask = (ustar == R(0));
   qint_iv1 = mask ? R(0.5) * (vl + vr) : qint_iv1;
   qint_iv2 = mask ? R(0.5) * (v2l + v2r) : qint_iv2;
-  // final Godunov state: star (spin >= 0), original (spout < 0) or the fan blend
-  const bool use_star = spin >= R(0);
-  const bool use_orig = !use_star && (spout < R(0));
-  const R qint_iu = use_star ? ustar : use_orig ? uo : frac * ustar + (R(1) - frac) * uo;
-  const R qint_gdpres = use_star ? pstar : use_orig ? po : frac * pstar + (R(1) - frac) * po;
+  const R sgnm = copysign(R(1), ustar);
+  R spout = co - sgnm * uo;
+  // final Godunov state: star (spin >= 0), original (spout < 0) or the fan blend, as
+  // cs * star + cn * original; rspo becomes its partial densities
+  R qint_iu = ustar, qint_gdpres = pstar, cs = R(1), cn = R(0);
+  if (!star_certain<MIX, R>(pabs(pstar, p0), rstar, ustar, pstar < po, spout)) {
+    const R cstar = ER::cs_w(rstar, pabs(pstar, p0), rspstar);
+    R spin = cstar - sgnm * ustar;
+    const R ushock = R(0.5) * (spin + spout);
+    mask = pstar < po;
+    spout = mask ? spout : ushock;
+    spin = mask ? spin : ushock;
+    if (!(spin >= R(0))) {
+      if (spout < R(0)) {
+        qint_iu = uo;
+        qint_gdpres = po;
+        cs = R(0);
+        cn = R(1);
+      } else {
+        const R scr = (fabs(spout - spin) < Lim<R>::very_small()) ? R(pcg::SMALL_NUM) * cav() : spout - spin;
+        const R frac = max0_min1<R>((R(1) + rdiv(spout + spin, scr)) * R(0.5));
+        qint_iu = frac * ustar + (R(1) - frac) * uo;
+        qint_gdpres = frac * pstar + (R(1) - frac) * po;
+        cs = frac;
+        cn = R(1) - frac;
+      }
+    }
+  }
   R rgd = R(0);
   if constexpr (sizeof(R) == 4 && NS > 1) {
-    const R cs = use_star ? R(1) : use_orig ? R(0) : frac;
-    const R cn = use_star ? R(0) : use_orig ? R(1) : R(1) - frac;
     rgd = blend2_sum<NS>(cs, rspstar, cn, rspo, rspo);
   } else {
 #pragma unroll
     for (int n = 0; n < NS; n++) {
-      rspo[n] = use_star ? rspstar[n] : use_orig ? rspo[n] : frac * rspstar[n] + (R(1) - frac) * rspo[n];
+      rspo[n] = cn == R(0) && cs == R(1) ? rspstar[n] : cs == R(0) && cn == R(1) ? rspo[n] : cs * rspstar[n] + cn * rspo[n];
       rgd += rspo[n];
     }
   }
@@ -822,8 +852,8 @@ __device__ __forceinline__ void riemann_reduced(const FaceState<NS, R>& L, const
   o.regd = regd;
 }
 
-template <int NS, bool MIX, class R>
-__device__ __forceinline__ void riemann(const FaceState<NS, R>& L, const FaceState<NS, R>& Rs, R cav,
+template <int NS, bool MIX, class R, class CAV>
+__device__ __forceinline__ void riemann(const FaceState<NS, R>& L, const FaceState<NS, R>& Rs, const CAV& cav,
                                         RiemannOut<R>& o) {
   using E = Eos<NS, MIX, R>;
   const R rl = L.rho, ul = L.un, vl = L.ut1, v2l = L.ut2, pl = L.p;
@@ -871,47 +901,43 @@ __device__ __forceinline__ void riemann(const FaceState<NS, R>& L, const FaceSta
     rspstar[n] = dmax(R(0), rspo[n] + drho * ytmp[n]);
     rstar += rspstar[n];
   }
-  div_all<NS>(rspstar, rstar, ytmp);
-  const R cstar = E::rpy2cs(rstar, pstar, ytmp);
-
   const R sgnm = copysign(R(1), ustar);
   R spout = co - sgnm * uo;
-  R spin = cstar - sgnm * ustar;
-  const R ushock = R(0.5) * (spin + spout);
-  mask = pstar < po;
-  spout = mask ? spout : ushock;
-  spin = mask ? spin : ushock;
-  const R scr = (fabs(spout - spin) < Lim<R>::very_small()) ? R(pcg::SMALL_NUM) * cav : spout - spin;
-  const R frac = max0_min1<R>((R(1) + (spout + spin) / scr) * R(0.5));
-
   mask = ustar > R(0);
   R qint_iv1 = mask ? vl : vr;
   R qint_iv2 = mask ? v2l : v2r;
   mask = (ustar == R(0));
   qint_iv1 = mask ? R(0.5) * (vl + vr) : qint_iv1;
   qint_iv2 = mask ? R(0.5) * (v2l + v2r) : qint_iv2;
-  R rspgd[NS];
+  // the Godunov state: star (spin >= 0), original (spout < 0) or the fan blend, its
+  // species in rspstar, their sum in rgd (the star state's sum is rstar)
+  R qint_iu = ustar, qint_gdpres = pstar, rgd = rstar;
+  div_all<NS>(rspstar, rstar, ytmp);
+  if (!star_certain<MIX, R>(pstar, rstar, ustar, pstar < po, spout)) {
+    const R cstar = E::rpy2cs(rstar, pstar, ytmp);
+    R spin = cstar - sgnm * ustar;
+    const R ushock = R(0.5) * (spin + spout);
+    mask = pstar < po;
+    spout = mask ? spout : ushock;
+    spin = mask ? spin : ushock;
+    if (!(spin >= R(0))) {
+      R frac = R(0);
+      const bool orig = spout < R(0);
+      if (!orig) {
+        const R scr = (fabs(spout - spin) < Lim<R>::very_small()) ? R(pcg::SMALL_NUM) * cav() : spout - spin;
+        frac = max0_min1<R>((R(1) + (spout + spin) / scr) * R(0.5));
+      }
+      qint_iu = orig ? uo : frac * ustar + (R(1) - frac) * uo;
+      qint_gdpres = orig ? po : frac * pstar + (R(1) - frac) * po;
+      rgd = R(0);
 #pragma unroll
-  for (int n = 0; n < NS; n++) rspgd[n] = frac * rspstar[n] + (R(1) - frac) * rspo[n];
-  R qint_iu = frac * ustar + (R(1) - frac) * uo;
-  R qint_gdpres = frac * pstar + (R(1) - frac) * po;
-
-  mask = (spout < R(0));
-#pragma unroll
-  for (int n = 0; n < NS; n++) rspgd[n] = mask ? rspo[n] : rspgd[n];
-  qint_iu = mask ? uo : qint_iu;
-  qint_gdpres = mask ? po : qint_gdpres;
-  mask = (spin >= R(0));
-  R rgd = R(0);
-#pragma unroll
-  for (int n = 0; n < NS; n++) {
-    rspgd[n] = mask ? rspstar[n] : rspgd[n];
-    rgd += rspgd[n];
+      for (int n = 0; n < NS; n++) {
+        rspstar[n] = orig ? rspo[n] : frac * rspstar[n] + (R(1) - frac) * rspo[n];
+        rgd += rspstar[n];
+      }
+      div_all<NS>(rspstar, rgd, ytmp);
+    }
   }
-  qint_iu = mask ? ustar : qint_iu;
-  qint_gdpres = mask ? pstar : qint_gdpres;
-
-  div_all<NS>(rspgd, rgd, ytmp);
   const R gdnv_e = E::ryp2e(rgd, ytmp, qint_gdpres);
   const R regd = rgd * gdnv_e;
 
@@ -937,9 +963,9 @@ __device__ __forceinline__ void riemann(const FaceState<NS, R>& L, const FaceSta
 // UMY, UMZ, UEDEN, UEINT and the species fluxes in absolute order. DIR is the normal.
 // With QX, qx[0..2] also receive the Godunov state's tangential velocities (t1, t2 in
 // absolute order) and rho*e, from which pc_umeth_3D's qint GDGAME is formed.
-template <int NS, bool MIX, bool EXACT, int DIR, class R, bool QX = false>
+template <int NS, bool MIX, bool EXACT, int DIR, class R, bool QX = false, class CAV>
 __device__ __forceinline__ void cmpflx(const R* ql, const R* qr, int idx, int bclo, int bchi, int domlo, int domhi,
-                                       R cav, R p0, R* fl, R& gun, R& gpres, R* qx = nullptr) {
+                                       const CAV& cav, R p0, R* fl, R& gun, R& gpres, R* qx = nullptr) {
   constexpr int t1 = (DIR == 0) ? 1 : 0;
   constexpr int t2 = (DIR == 2) ? 1 : 2;
   FaceState<NS, R> L, Rs;

@@ -1068,9 +1068,58 @@ int pcg_set_eos_gamma(double gamma, double mw) {
   c.gamma = gamma;
   c.imw[0] = 1.0 / mw;
   c.gammaf = (float)gamma;
+  // cv > 0 everywhere: only p / rho that neither under- nor overflows
+  c.star_lo = c.star_lof = 1e-30f;
+  c.star_hi = c.star_hif = 1e30f;
   c.imwf[0] = (float)c.imw[0];
   return store_eos(0, c);
 }
+
+}  // extern "C"
+
+namespace {
+
+// Whether cv of the polynomial c (5 coefficients) is positive on [t, t + h], by more than
+// FP32 rounding of its terms: its value at t against the largest change over h.
+bool cv_positive(const double* c, double t, double h) {
+  double v = 0.0, mag = 0.0, slope = 0.0, p = 1.0;
+  const double te = t + h;
+  for (int i = 0; i < 5; ++i) {
+    v += c[i] * p;
+    p *= t;
+    mag += std::fabs(c[i]) * std::pow(te, i);
+    if (i) slope += std::fabs(c[i]) * i * std::pow(te, i - 1);
+  }
+  return v - slope * h > 1e-4 * mag;
+}
+
+// EosConst::star_lo/hi of a mixture table: the widest temperature range around the
+// species' range switches (scanned in 1 K steps, up to 20000 K) in which every cv_k is
+// positive, as bounds on p / rho = RU T sum(Y / W) that hold for any composition.
+void star_bounds(pcg::EosConst& c) {
+  double lo = 0.0, hi = 20000.0, wmin = 1.0 / c.imw[0], wmax = wmin;
+  for (int k = 0; k < c.nspec; ++k) {
+    wmin = std::min(wmin, 1.0 / c.imw[k]);
+    wmax = std::max(wmax, 1.0 / c.imw[k]);
+    // the switch clamped to the scanned range (a NaN switch always takes the upper range)
+    const double tm = c.tmid[k] > 0.0 ? std::min(c.tmid[k], 20000.0) : 0.0;
+    double t = tm;
+    while (t < hi && cv_positive(c.cvc[k][1], t, 1.0)) t += 1.0;
+    hi = std::min(hi, t);
+    t = tm;
+    while (t > lo && cv_positive(c.cvc[k][0], std::max(t - 1.0, 0.0), 1.0)) t -= 1.0;
+    lo = std::max(lo, t);
+  }
+  lo = std::max(lo, 1e-3);
+  c.star_lo = lo * pcg::RU / wmin * (1.0 + 1e-5);
+  c.star_hi = hi * pcg::RU / wmax * (1.0 - 1e-5);
+  c.star_lof = (float)c.star_lo;
+  c.star_hif = (float)c.star_hi;
+}
+
+}  // namespace
+
+extern "C" {
 
 int pcg_set_eos_nasa7(int nspec, const double* mw, const double* tmid, const double* a_lo, const double* a_hi) {
   if (nspec < 2 || nspec > pcg::MAXNS) return fail(PCG_EINVAL, "nspec must be in 2..%d", pcg::MAXNS);
@@ -1107,6 +1156,7 @@ int pcg_set_eos_nasa7(int nspec, const double* mw, const double* tmid, const dou
     c.imwf[k] = c.imwp[k] = (float)c.imw[k];
     c.tmidf[k] = (float)c.tmid[k];
   }
+  star_bounds(c);
   return store_eos(1, c);
 }
 

@@ -869,9 +869,11 @@ __device__ __forceinline__ void load_state(const C& t, R* s) {
 template <int NS, bool MIX, bool EXACT, int D, class R, bool QX = false>
 __device__ __forceinline__ void face_flux(const pcg::Region& rg, int i, int j, int k, const R* ql, const R* qr,
                                           R p0, R* fl, R& gun, R& gpres, R* qx = nullptr) {
-  const V4<const double> qav = v4<const double>(rg.qa);
-  const CellPtr<const double> qa = at(qav, i, j, k);
-  const R cav = R(0.5 * (qa[pcg::QC] + qa.p[-dstride(qav, D) + pcg::QC * qa.ns]));
+  const auto cav = [&] {  // read by fans of zero width only
+    const V4<const double> qav = v4<const double>(rg.qa);
+    const CellPtr<const double> qa = at(qav, i, j, k);
+    return R(0.5 * (qa[pcg::QC] + qa.p[-dstride(qav, D) + pcg::QC * qa.ns]));
+  };
   const int idx = (D == 0) ? i : (D == 1) ? j : k;
   cmpflx<NS, MIX, EXACT, D, R, QX>(ql, qr, idx, rg.bclo[D], rg.bchi[D], rg.domlo[D], rg.domhi[D], cav, p0, fl, gun,
                                    gpres, qx);

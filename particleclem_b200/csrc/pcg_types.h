@@ -58,11 +58,15 @@ struct EosConst {
   int nspec;
   int uniform_tmid;  // 1: every species switches NASA-7 range at tmid[0]
   double gamma;
+  // bounds on p / rho (any composition) within which cv of every species is positive, and
+  // so the sound speed above sqrt(p / rho): see star_certain (pcg_device.cuh)
+  double star_lo, star_hi;
   double imw[MAXNS];
   double tmid[MAXNS];
   double cvc[MAXNS][2][5];
   double ec[MAXNS][2][6];
   float gammaf;
+  float star_lof, star_hif;
   float imwf[MAXNS];
   float tmidf[MAXNS];
   float cvcf[MAXNS][2][5];
