@@ -3,6 +3,8 @@
 // ghost fill. All FP64.
 #pragma once
 
+#include <cooperative_groups.h>
+
 #include "pcg_kernels.cuh"
 
 namespace PCG_TU {
@@ -82,12 +84,41 @@ __global__ void __launch_bounds__(128) k_estdt(pcg::AuxArgs a) {
   if (threadIdx.x == 0) a.partial[blockIdx.x] = dt;
 }
 
-// Final reduction of the block minima, then estdt_hydro *= cfl (Source/PeleC.cpp:930).
-__global__ void __launch_bounds__(128) k_estdt_final(pcg::AuxArgs a) {
+// Final reduction of the block minima, then estdt_hydro *= cfl (Source/PeleC.cpp:930), by one
+// cluster of up to 8 blocks of 1024 threads (host: one block per 4096 minima), four loads in
+// flight per thread; block 0 gathers the blocks' minima from their shared memory. The
+// launch is a chain of load latencies, not bandwidth: one block of 128 threads took 21 us
+// for the 16384 minima of a 128^3 level, as many loads in turn as this takes passes.
+constexpr int kFinalThreads = 1024, kFinalLoads = 4, kFinalBlocks = 8;
+__global__ void __launch_bounds__(kFinalThreads) k_estdt_final(pcg::AuxArgs a) {
+  namespace cg = cooperative_groups;
+  __shared__ double sh[kFinalThreads / 32], part;
+  const cg::cluster_group cl = cg::this_cluster();
+  const int64_t stride = int64_t(gridDim.x) * kFinalThreads;
   double v = DBL_MAX;
-  for (int64_t b = threadIdx.x; b < a.npartial; b += blockDim.x) v = dmin(v, a.partial[b]);
-  v = block_min(v);
-  if (threadIdx.x == 0) *a.dt_out = v * a.cfl;
+  for (int64_t b = int64_t(blockIdx.x) * kFinalThreads + threadIdx.x; b < a.npartial; b += kFinalLoads * stride) {
+    double w[kFinalLoads];
+#pragma unroll
+    for (int m = 0; m < kFinalLoads; ++m) w[m] = b + m * stride < a.npartial ? a.partial[b + m * stride] : DBL_MAX;
+#pragma unroll
+    for (int m = 0; m < kFinalLoads; ++m) v = dmin(v, w[m]);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = dmin(v, __shfl_xor_sync(0xffffffffu, v, o));
+  if (threadIdx.x % 32 == 0) sh[threadIdx.x / 32] = v;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    v = sh[threadIdx.x];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = dmin(v, __shfl_xor_sync(0xffffffffu, v, o));
+    if (threadIdx.x == 0) part = v;
+  }
+  cl.sync();
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    for (unsigned r = 1; r < cl.num_blocks(); ++r) v = dmin(v, *cl.map_shared_rank(&part, r));
+    *a.dt_out = v * a.cfl;
+  }
+  cl.sync();  // the minima stay readable until block 0 is done
 }
 
 // Source/Advance.cpp:397-417 (construct_Snew, hydro only) then Source/PeleC.cpp:2289-2305
@@ -185,38 +216,52 @@ __device__ __forceinline__ int ghost_src(int c, int lo, int hi, bool periodic) {
   return c;
 }
 // Ghost cell number t of the domain [dlo, dhi] grown by ng (t < the ghost-cell count) gets
-// its value from the valid cell the fill maps it to; false when t is past the last ghost.
-__device__ __forceinline__ bool fill_ghost(int64_t t, const int* dlo, const int* dhi, int ng, int periodic,
-                                          const pcg::View& state, int ncomp) {
-  const int n0 = dhi[0] - dlo[0] + 1, n1 = dhi[1] - dlo[1] + 1, n2 = dhi[2] - dlo[2] + 1;
-  const int64_t e0 = n0 + 2 * ng, e1 = n1 + 2 * ng;
-  const int64_t cz = e0 * e1 * 2 * ng, cy = e0 * 2 * ng * n2, cx = (int64_t)2 * ng * n1 * n2;
+// its value from the valid cell the fill maps it to; a t past the last ghost cell does nothing.
+// Eight components are loaded before any is stored (no ghost cell is a source): copied one by
+// one, each component waits out the load before it, 16 of them 30 us on a 128^3 level.
+// A view spans fewer than 2^31 elements, so the cell numbers are 32-bit.
+__device__ __forceinline__ void fill_ghost(unsigned t, const int* dlo, const int* dhi, int ng, int periodic,
+                                           const pcg::View& state, int ncomp) {
+  const unsigned n0 = dhi[0] - dlo[0] + 1, n1 = dhi[1] - dlo[1] + 1, n2 = dhi[2] - dlo[2] + 1;
+  const unsigned g2 = 2 * ng, e0 = n0 + g2, e1 = n1 + g2;
+  const unsigned cz = e0 * e1 * g2, cy = e0 * g2 * n2, cx = g2 * n1 * n2;
   int c[3];
   if (t < cz) {  // z ghost slabs: (i, j) over the grown extent, 2 ng layers
-    const int g = (int)(t / (e0 * e1));
-    c[0] = (int)(t % e0) + dlo[0] - ng;
-    c[1] = (int)((t / e0) % e1) + dlo[1] - ng;
+    const unsigned r = t / e0;
+    const int g = (int)(r / e1);
+    c[0] = (int)(t - r * e0) + dlo[0] - ng;
+    c[1] = (int)(r % e1) + dlo[1] - ng;
     c[2] = (g < ng) ? dlo[2] - ng + g : dhi[2] + 1 + (g - ng);
   } else if (t < cz + cy) {  // y ghost slabs of the valid k
-    const int64_t u = t - cz;
-    const int g = (int)((u / e0) % (2 * ng));
-    c[0] = (int)(u % e0) + dlo[0] - ng;
+    const unsigned u = t - cz, r = u / e0;
+    const int g = (int)(r % g2);
+    c[0] = (int)(u - r * e0) + dlo[0] - ng;
     c[1] = (g < ng) ? dlo[1] - ng + g : dhi[1] + 1 + (g - ng);
-    c[2] = (int)(u / (e0 * 2 * ng)) + dlo[2];
+    c[2] = (int)(r / g2) + dlo[2];
   } else if (t < cz + cy + cx) {  // x ghost slabs of the valid (j, k)
-    const int64_t u = t - cz - cy;
-    const int g = (int)(u % (2 * ng));
+    const unsigned u = t - cz - cy, r = u / g2;
+    const int g = (int)(u - r * g2);
     c[0] = (g < ng) ? dlo[0] - ng + g : dhi[0] + 1 + (g - ng);
-    c[1] = (int)((u / (2 * ng)) % n1) + dlo[1];
-    c[2] = (int)(u / ((int64_t)2 * ng * n1)) + dlo[2];
+    c[1] = (int)(r % n1) + dlo[1];
+    c[2] = (int)(r / n1) + dlo[2];
   } else {
-    return false;
+    return;
   }
   int src[3];
   for (int d = 0; d < 3; ++d) src[d] = ghost_src(c[d], dlo[d], dhi[d], (periodic >> d) & 1);
   const V4<double> s = v4<double>(state);
-  for (int comp = 0; comp < ncomp; ++comp) s(c[0], c[1], c[2], comp) = s(src[0], src[1], src[2], comp);
-  return true;
+  const double* from = &s(src[0], src[1], src[2], 0);
+  double* to = &s(c[0], c[1], c[2], 0);
+  constexpr int B = 8;
+  for (int comp = 0; comp < ncomp; comp += B) {
+    double v[B];
+#pragma unroll
+    for (int m = 0; m < B; ++m)
+      if (comp + m < ncomp) v[m] = from[(comp + m) * s.ns];
+#pragma unroll
+    for (int m = 0; m < B; ++m)
+      if (comp + m < ncomp) to[(comp + m) * s.ns] = v[m];
+  }
 }
 
 // The ghost cells of many independent boxes (each its own domain) in one launch: the
@@ -229,8 +274,8 @@ __global__ void __launch_bounds__(128) k_fill_boxes(pcg::AuxArgs a) {
     if (a.fills[mid].blk0 <= blk) lo = mid; else hi = mid - 1;
   }
   const pcg::FillBox& f = a.fills[lo];
-  const int64_t t = (blk - f.blk0) * blockDim.x + threadIdx.x;
-  if (t >= f.count) return;
+  const unsigned t = unsigned(blk - f.blk0) * blockDim.x + threadIdx.x;
+  if (t >= (unsigned)f.count) return;
   fill_ghost(t, f.dlo, f.dhi, a.ng, f.periodic, f.state, a.ncomp);
 }
 
@@ -260,7 +305,7 @@ __global__ void __launch_bounds__(128) k_copy_box(pcg::AuxArgs a) {
 }
 
 __global__ void __launch_bounds__(128) k_fill(pcg::AuxArgs a) {
-  fill_ghost((int64_t)blockIdx.x * blockDim.x + threadIdx.x, a.dlo, a.dhi, a.ng, a.periodic, a.state, a.ncomp);
+  fill_ghost(blockIdx.x * blockDim.x + threadIdx.x, a.dlo, a.dhi, a.ng, a.periodic, a.state, a.ncomp);
 }
 
 template <int NS, bool MIX>
@@ -276,13 +321,28 @@ static cudaError_t launch_advance_t(const pcg::StageArgs& a, int64_t nblocks, in
   return cudaGetLastError();
 }
 
+static cudaError_t launch_estdt_final(const pcg::AuxArgs& a, cudaStream_t s) {
+  const int64_t want = (a.npartial + kFinalThreads * kFinalLoads - 1) / (kFinalThreads * kFinalLoads);
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = unsigned(want < 1 ? 1 : want > kFinalBlocks ? kFinalBlocks : want);
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(at.val.clusterDim.x);
+  cfg.blockDim = dim3(kFinalThreads);
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_estdt_final, a);
+}
+
 template <int NS, bool MIX>
 static cudaError_t launch_aux_t(int which, const pcg::AuxArgs& a, int64_t nblocks, cudaStream_t s) {
   if (nblocks <= 0) return cudaSuccess;
   const dim3 grid((unsigned)nblocks), block(128);
   switch (which) {
     case AUX_ESTDT: k_estdt<NS, MIX><<<grid, block, 0, s>>>(a); break;
-    case AUX_ESTDT_FINAL: k_estdt_final<<<1, block, 0, s>>>(a); break;
+    case AUX_ESTDT_FINAL: return launch_estdt_final(a, s);
     case AUX_UPDATE: k_update<NS, MIX><<<grid, block, 0, s>>>(a); break;
     case AUX_FILL: k_fill<<<grid, block, 0, s>>>(a); break;
     case AUX_FILL_BOXES: k_fill_boxes<<<grid, block, 0, s>>>(a); break;
