@@ -385,21 +385,23 @@ struct Eos {
     }
     dpdr_e = rm * t;
   }
-  // RTY2P, RTY2Cs, RTY2G and RTY2dpde_dpdre of one state, sharing rmix and cv: each
-  // value is formed by exactly the operations of the separate calls.
-  static __device__ __forceinline__ void rty2all(R r, R t, const R* y, R& p, R& cs, R& g, R& dpde, R& dpdr_e) {
-    const R rm = rmix(y);
+  // RTY2P, RTY2Cs and RTY2G of one state, sharing rmix and cv (left in rm, cv for
+  // dpde_dpdre): each value is formed by exactly the operations of the separate calls.
+  static __device__ __forceinline__ void rty2pcg(R r, R t, const R* y, R& p, R& cs, R& g, R& rm, R& cv) {
+    rm = rmix(y);
     p = r * rm * t;
     if (!MIX) {
+      cv = R(0);
       g = C::gamma();
       cs = sqrt(C::gamma() * p / r);
-      dpde = (C::gamma() - R(1)) * r;
     } else {
-      const R cv = cv_of(t, y);
+      cv = cv_of(t, y);
       g = (cv + rm) / cv;
       cs = sqrt(g * p / r);
-      dpde = r * rm / cv;
     }
+  }
+  static __device__ __forceinline__ void dpde_dpdre(R r, R t, R rm, R cv, R& dpde, R& dpdr_e) {
+    dpde = MIX ? r * rm / cv : (C::gamma() - R(1)) * r;
     dpdr_e = rm * t;
   }
   static __device__ __forceinline__ R y2wbar(const R* y) {

@@ -611,6 +611,7 @@ void build_layout(Layout& L, const std::vector<BoxIn>& boxes, const pcg_hydro_pa
       // the mixed form keeps no FP64 primitive array: its stages read the FP32 copy
       if (!single) take(L, g4, nq, 8, R.q);
       take(L, g4, pcg::NQAUX, 8, R.qa);
+      R.stage_q = 1;
       add_seg(L, K_CTOPRIM, (int)r, 0, g4);
     } else {
       R.q = B.q;

@@ -171,10 +171,9 @@ __global__ void __launch_bounds__(128, MINB) k_ctoprim(pcg::StageArgs a) {
   for (int n = 0; n < NS; n++)
     if ((-1e-4 * DBL_EPSILON < y[n]) && (y[n] < 1e-4 * DBL_EPSILON)) y[n] = 0.0;
   const double e = (u[pcg::UEDEN] - kineng) * rhoinv;
-  const double wbar = E::y2wbar(y);
   const double T = E::rey2t(e, y, u[pcg::UTEMP]);
-  double p, cs, gam1, dpde, dpdr_e;
-  E::rty2all(rho, T, y, p, cs, gam1, dpde, dpdr_e);
+  double p, cs, gam1, rm, cv;
+  E::rty2pcg(rho, T, y, p, cs, gam1, rm, cv);
   // the FP64 primitive array exists in the FP64 forms; the mixed form's stages read the
   // FP32 copy below instead
   if (rg.q.p) {
@@ -185,17 +184,24 @@ __global__ void __launch_bounds__(128, MINB) k_ctoprim(pcg::StageArgs a) {
     q[pcg::QW] = vz;
 #pragma unroll
     for (int n = 0; n < NS; n++) q[pcg::QFS + n] = y[n];
-    q[pcg::QTEMP] = T;
     q[pcg::QREINT] = e * rho;
     q[pcg::QPRES] = p;
-    q[pcg::QGAME] = p / (e * rho) + 1.0;
+    if (!rg.stage_q) {
+      q[pcg::QTEMP] = T;
+      q[pcg::QGAME] = p / (e * rho) + 1.0;
+    }
   }
-  qa[pcg::QDPDR] = dpdr_e;
-  qa[pcg::QDPDE] = dpde;
   qa[pcg::QGAMC] = gam1;
   qa[pcg::QC] = cs;
-  qa[pcg::QCSML] = dmax(pcg::SMALL_NUM, pcg::SMALL_NUM * cs);
-  qa[pcg::QRSPEC] = pcg::RU / wbar;
+  // what no stage of the advance reads: only for a caller's q and qaux (pcg_ctoprim)
+  if (!rg.stage_q) {
+    double dpde, dpdr_e;
+    E::dpde_dpdre(rho, T, rm, cv, dpde, dpdr_e);
+    qa[pcg::QDPDR] = dpdr_e;
+    qa[pcg::QDPDE] = dpde;
+    qa[pcg::QCSML] = dmax(pcg::SMALL_NUM, pcg::SMALL_NUM * cs);
+    qa[pcg::QRSPEC] = pcg::RU / E::y2wbar(y);
+  }
   // mixed form: the FP32 primitive copy the trace reads, on grow(box, qf_grow)
   const int gq = rg.qf_grow;
   if (rg.qf.p && !rg.qf_in_prep && it.i >= rg.lo[0] - gq && it.i <= rg.hi[0] + gq && it.j >= rg.lo[1] - gq &&

@@ -130,7 +130,10 @@ struct Region {
   // (the caller's NGDNV-component arrays, GDRHO untouched), and p div u goes to pdivu
   // instead of the flux divergence
   int32_t umeth;
-  int32_t pad2;
+  // 1: q and qa are workspace arrays that only the stages read, so k_ctoprim leaves out the
+  // components no stage reads (T, QGAME, QCSML, dp/dr, dp/de, QRSPEC: three divisions and
+  // six stores per cell of grow(box,4))
+  int32_t stage_q;
   View pdivu;       // umeth: p div u on the box, double
   View src;         // pcg_srctoprim: conserved sources, double, NVAR comps
 };
