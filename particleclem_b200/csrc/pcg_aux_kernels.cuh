@@ -12,14 +12,8 @@ namespace PCG_TU {
 enum { AUX_ESTDT = 0, AUX_ESTDT_FINAL, AUX_UPDATE, AUX_FILL, AUX_FILL_BOXES, AUX_ESTDT_BOXES, AUX_COPY };
 
 __device__ __forceinline__ bool aux_item(const pcg::AuxArgs& a, const pcg::AuxBox*& bx, int& i, int& j, int& k) {
-  const int blk = blockIdx.x;
-  int lo = 0, hi = a.nseg - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (a.segs[mid].blk0 <= blk) lo = mid; else hi = mid - 1;
-  }
-  const pcg::Seg& s = a.segs[lo];
-  const unsigned local = unsigned(blk - (int)s.blk0) * blockDim.x + threadIdx.x;
+  const pcg::Seg s = find_seg(a.few, a.segs, a.nseg, a.overlap);
+  const unsigned local = unsigned(int(blockIdx.x) - (int)s.blk0) * blockDim.x + threadIdx.x;
   if (local >= (unsigned)s.count) return false;
   const unsigned n0 = s.n[0], n1 = s.n[1];
   const unsigned t = local / n0;
@@ -69,7 +63,7 @@ __device__ __forceinline__ double cfl_dt(const double* s, const double* dx) {
 
 // Per-cell CFL constraints of every valid cell, block minima.
 template <int NS, bool MIX>
-__global__ void __launch_bounds__(128) k_estdt(pcg::AuxArgs a) {
+__global__ void __launch_bounds__(128) k_estdt(const __grid_constant__ pcg::AuxArgs a) {
   const pcg::AuxBox* bx;
   int i, j, k;
   double dt = DBL_MAX;
@@ -90,11 +84,12 @@ __global__ void __launch_bounds__(128) k_estdt(pcg::AuxArgs a) {
 // launch is a chain of load latencies, not bandwidth: one block of 128 threads took 21 us
 // for the 16384 minima of a 128^3 level, as many loads in turn as this takes passes.
 constexpr int kFinalThreads = 1024, kFinalLoads = 4, kFinalBlocks = 8;
-__global__ void __launch_bounds__(kFinalThreads) k_estdt_final(pcg::AuxArgs a) {
+__global__ void __launch_bounds__(kFinalThreads) k_estdt_final(const __grid_constant__ pcg::AuxArgs a) {
   namespace cg = cooperative_groups;
   __shared__ double sh[kFinalThreads / 32], part;
   const cg::cluster_group cl = cg::this_cluster();
   const int64_t stride = int64_t(gridDim.x) * kFinalThreads;
+  await_previous(a.overlap);
   double v = DBL_MAX;
   for (int64_t b = int64_t(blockIdx.x) * kFinalThreads + threadIdx.x; b < a.npartial; b += kFinalLoads * stride) {
     double w[kFinalLoads];
@@ -152,7 +147,7 @@ __device__ __forceinline__ void update_cell(double* s, const double* hsrc, doubl
 }
 
 template <int NS, bool MIX>
-__global__ void __launch_bounds__(128) k_update(pcg::AuxArgs a) {
+__global__ void __launch_bounds__(128) k_update(const __grid_constant__ pcg::AuxArgs a) {
   const pcg::AuxBox* bx;
   int i, j, k;
   if (!aux_item(a, bx, i, j, k)) return;
@@ -178,7 +173,7 @@ __global__ void __launch_bounds__(128) k_update(pcg::AuxArgs a) {
 // minimum is k_estdt_final). Each value is formed by the same expressions as k_consup,
 // k_update and k_estdt, so the step is the unfused step's.
 template <int NS, bool MIX, int MINB>
-__global__ void __launch_bounds__(128, MINB) k_advance(pcg::StageArgs a) {
+__global__ void __launch_bounds__(128, MINB) k_advance(const __grid_constant__ pcg::StageArgs a) {
   Item it;
   double dtc = DBL_MAX;
   if (item_of(a, it)) {
@@ -266,7 +261,8 @@ __device__ __forceinline__ void fill_ghost(unsigned t, const int* dlo, const int
 
 // The ghost cells of many independent boxes (each its own domain) in one launch: the
 // block finds its box by binary search over the boxes' first blocks.
-__global__ void __launch_bounds__(128) k_fill_boxes(pcg::AuxArgs a) {
+__global__ void __launch_bounds__(128) k_fill_boxes(const __grid_constant__ pcg::AuxArgs a) {
+  await_previous(a.overlap);
   const int64_t blk = blockIdx.x;
   int lo = 0, hi = a.nfill - 1;
   while (lo < hi) {
@@ -282,7 +278,8 @@ __global__ void __launch_bounds__(128) k_fill_boxes(pcg::AuxArgs a) {
 // The next timestep of every box of a batched step: block b reduces the CFL minima the
 // fused tail left for region b (the blocks of its advance segment), times cfl, into
 // dt_boxes[b].
-__global__ void __launch_bounds__(128) k_estdt_boxes(pcg::AuxArgs a) {
+__global__ void __launch_bounds__(128) k_estdt_boxes(const __grid_constant__ pcg::AuxArgs a) {
+  await_previous(a.overlap);
   const pcg::Seg& sg = a.bsegs[blockIdx.x];
   const int64_t nb = (sg.count + 127) / 128;
   double v = DBL_MAX;
@@ -293,7 +290,8 @@ __global__ void __launch_bounds__(128) k_estdt_boxes(pcg::AuxArgs a) {
 
 // Copy of the cells [dlo, dhi] of every component from one device FAB (state) to another
 // (dst), FP64: the packing and unpacking of halo planes. One thread per cell and component.
-__global__ void __launch_bounds__(128) k_copy_box(pcg::AuxArgs a) {
+__global__ void __launch_bounds__(128) k_copy_box(const __grid_constant__ pcg::AuxArgs a) {
+  await_previous(a.overlap);
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t n0 = a.dhi[0] - a.dlo[0] + 1, n1 = a.dhi[1] - a.dlo[1] + 1, n2 = a.dhi[2] - a.dlo[2] + 1;
   const int64_t cells = n0 * n1 * n2;
@@ -304,53 +302,43 @@ __global__ void __launch_bounds__(128) k_copy_box(pcg::AuxArgs a) {
   v4<double>(a.dst)(i, j, k, comp) = v4<const double>(a.state)(i, j, k, comp);
 }
 
-__global__ void __launch_bounds__(128) k_fill(pcg::AuxArgs a) {
+__global__ void __launch_bounds__(128) k_fill(const __grid_constant__ pcg::AuxArgs a) {
+  await_previous(a.overlap);
   fill_ghost(blockIdx.x * blockDim.x + threadIdx.x, a.dlo, a.dhi, a.ng, a.periodic, a.state, a.ncomp);
+}
+
+static cudaError_t launch_estdt_final(const pcg::AuxArgs& a, cudaStream_t s) {
+  const int64_t want = (a.npartial + kFinalThreads * kFinalLoads - 1) / (kFinalThreads * kFinalLoads);
+  const unsigned nb = unsigned(want < 1 ? 1 : want > kFinalBlocks ? kFinalBlocks : want);
+  return launch_kernel(k_estdt_final, nb, kFinalThreads, nb, a, s);
 }
 
 template <int NS, bool MIX>
 static cudaError_t launch_advance_t(const pcg::StageArgs& a, int64_t nblocks, int variant, cudaStream_t s) {
   if (nblocks <= 0) return cudaSuccess;
-  const dim3 grid((unsigned)nblocks), block(128);
+  const unsigned grid = (unsigned)nblocks;
   switch (variant) {
-    case 0: k_advance<NS, MIX, kMinBlocks[K_CONSUP][0]><<<grid, block, 0, s>>>(a); break;
-    case 1: k_advance<NS, MIX, kMinBlocks[K_CONSUP][1]><<<grid, block, 0, s>>>(a); break;
-    case 2: k_advance<NS, MIX, kMinBlocks[K_CONSUP][2]><<<grid, block, 0, s>>>(a); break;
+    case 0: return launch_kernel(k_advance<NS, MIX, kMinBlocks[K_CONSUP][0]>, grid, a, s);
+    case 1: return launch_kernel(k_advance<NS, MIX, kMinBlocks[K_CONSUP][1]>, grid, a, s);
+    case 2: return launch_kernel(k_advance<NS, MIX, kMinBlocks[K_CONSUP][2]>, grid, a, s);
     default: return cudaErrorInvalidValue;
   }
-  return cudaGetLastError();
-}
-
-static cudaError_t launch_estdt_final(const pcg::AuxArgs& a, cudaStream_t s) {
-  const int64_t want = (a.npartial + kFinalThreads * kFinalLoads - 1) / (kFinalThreads * kFinalLoads);
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = unsigned(want < 1 ? 1 : want > kFinalBlocks ? kFinalBlocks : want);
-  at.val.clusterDim.y = at.val.clusterDim.z = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(at.val.clusterDim.x);
-  cfg.blockDim = dim3(kFinalThreads);
-  cfg.stream = s;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_estdt_final, a);
 }
 
 template <int NS, bool MIX>
 static cudaError_t launch_aux_t(int which, const pcg::AuxArgs& a, int64_t nblocks, cudaStream_t s) {
   if (nblocks <= 0) return cudaSuccess;
-  const dim3 grid((unsigned)nblocks), block(128);
+  const unsigned grid = (unsigned)nblocks;
   switch (which) {
-    case AUX_ESTDT: k_estdt<NS, MIX><<<grid, block, 0, s>>>(a); break;
+    case AUX_ESTDT: return launch_kernel(k_estdt<NS, MIX>, grid, a, s);
     case AUX_ESTDT_FINAL: return launch_estdt_final(a, s);
-    case AUX_UPDATE: k_update<NS, MIX><<<grid, block, 0, s>>>(a); break;
-    case AUX_FILL: k_fill<<<grid, block, 0, s>>>(a); break;
-    case AUX_FILL_BOXES: k_fill_boxes<<<grid, block, 0, s>>>(a); break;
-    case AUX_ESTDT_BOXES: k_estdt_boxes<<<grid, block, 0, s>>>(a); break;
-    case AUX_COPY: k_copy_box<<<grid, block, 0, s>>>(a); break;
+    case AUX_UPDATE: return launch_kernel(k_update<NS, MIX>, grid, a, s);
+    case AUX_FILL: return launch_kernel(k_fill, grid, a, s);
+    case AUX_FILL_BOXES: return launch_kernel(k_fill_boxes, grid, a, s);
+    case AUX_ESTDT_BOXES: return launch_kernel(k_estdt_boxes, grid, a, s);
+    case AUX_COPY: return launch_kernel(k_copy_box, grid, a, s);
     default: return cudaErrorInvalidValue;
   }
-  return cudaGetLastError();
 }
 
 }  // namespace PCG_TU

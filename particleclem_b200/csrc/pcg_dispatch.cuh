@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 
 #include "pcg_kernels.cuh"
+#include "pcg_launch.cuh"
 #include "pcg_aux_kernels.cuh"
 #include "pcg_units.h"
 
@@ -32,52 +33,47 @@ constexpr bool kExact = false;  // reduced algebra
 #endif
 
 template <int NS, bool MIX, class R, int V>
-static cudaError_t launch_v(int stage, const pcg::StageArgs& a, const dim3& grid, const dim3& block, cudaStream_t s) {
+static cudaError_t launch_v(int stage, const pcg::StageArgs& a, unsigned grid, cudaStream_t s) {
   switch (stage) {
-    case K_CTOPRIM: k_ctoprim<NS, MIX, kMinBlocks[K_CTOPRIM][V]><<<grid, block, 0, s>>>(a); break;
-    case K_PREP: k_prep<NS, MIX, kExact, R><<<grid, block, 0, s>>>(a); break;
+    case K_CTOPRIM: return launch_kernel(k_ctoprim<NS, MIX, kMinBlocks[K_CTOPRIM][V]>, grid, a, s);
+    case K_PREP: return launch_kernel(k_prep<NS, MIX, kExact, R>, grid, a, s);
     case K_TRACE:
       if (a.use_hybrid_weno && a.ppm_type == 1)
-        k_trace_weno<NS, MIX, kExact, R><<<grid, block, 0, s>>>(a);  // one shape for every variant
-      else
-        k_trace<NS, MIX, kExact, R, kMinBlocks[K_TRACE][V]><<<grid, block, 0, s>>>(a);
-      break;
-    case K_FLUX0: k_flux0<NS, MIX, kExact, R, kMinBlocks[K_FLUX0][V]><<<grid, block, 0, s>>>(a); break;
-    case K_FLUX1: k_flux1<NS, MIX, kExact, R, kMinBlocks[K_FLUX1][V]><<<grid, block, 0, s>>>(a); break;
-    case K_FLUX2: k_flux2<NS, MIX, kExact, R, kMinBlocks[K_FLUX2][V]><<<grid, block, 0, s>>>(a); break;
-    case K_CONSUP: k_consup<NS, MIX><<<grid, block, 0, s>>>(a); break;
-    case K_LOWBC: k_lowbc<NS, MIX, kExact, R><<<grid, block, 0, s>>>(a); break;
+        return launch_kernel(k_trace_weno<NS, MIX, kExact, R>, grid, a, s);  // one shape for every variant
+      return launch_kernel(k_trace<NS, MIX, kExact, R, kMinBlocks[K_TRACE][V]>, grid, a, s);
+    case K_FLUX0: return launch_kernel(k_flux0<NS, MIX, kExact, R, kMinBlocks[K_FLUX0][V]>, grid, a, s);
+    case K_FLUX1: return launch_kernel(k_flux1<NS, MIX, kExact, R, kMinBlocks[K_FLUX1][V]>, grid, a, s);
+    case K_FLUX2: return launch_kernel(k_flux2<NS, MIX, kExact, R, kMinBlocks[K_FLUX2][V]>, grid, a, s);
+    case K_CONSUP: return launch_kernel(k_consup<NS, MIX>, grid, a, s);
+    case K_LOWBC: return launch_kernel(k_lowbc<NS, MIX, kExact, R>, grid, a, s);
     default: return cudaErrorInvalidValue;
   }
-  return cudaGetLastError();
 }
 
 // pcg_umeth's final stage (raw fluxes and face states), its low-order boundary faces and
 // p div u; pcg_srctoprim. One launch shape each.
 template <int NS, bool MIX, class R>
-static cudaError_t launch_special(int stage, const pcg::StageArgs& a, const dim3& grid, const dim3& block,
+static cudaError_t launch_special(int stage, const pcg::StageArgs& a, unsigned grid,
                                   cudaStream_t s) {
   switch (stage) {
-    case K_FLUX2: k_flux2<NS, MIX, kExact, R, 0, true><<<grid, block, 0, s>>>(a); break;
-    case K_LOWBC: k_lowbc<NS, MIX, kExact, R, true><<<grid, block, 0, s>>>(a); break;
-    case K_CONSUP: k_pdivu<NS><<<grid, block, 0, s>>>(a); break;
-    case K_SRCQ: k_srctoprim<NS><<<grid, block, 0, s>>>(a); break;
+    case K_FLUX2: return launch_kernel(k_flux2<NS, MIX, kExact, R, 0, true>, grid, a, s);
+    case K_LOWBC: return launch_kernel(k_lowbc<NS, MIX, kExact, R, true>, grid, a, s);
+    case K_CONSUP: return launch_kernel(k_pdivu<NS>, grid, a, s);
+    case K_SRCQ: return launch_kernel(k_srctoprim<NS>, grid, a, s);
     default: return cudaErrorInvalidValue;
   }
-  return cudaGetLastError();
 }
 
 template <int NS, bool MIX, class R>
-static cudaError_t launch_trace_tile(const pcg::StageArgs& a, const dim3& grid, const dim3& block, int variant,
+static cudaError_t launch_trace_tile(const pcg::StageArgs& a, unsigned grid, int variant,
                                     cudaStream_t s) {
   if constexpr (sizeof(R) == 4 && pcg::trace_tile_species(NS)) {
     switch (variant) {
-      case 0: k_trace_tile<NS, MIX, kMinBlocks[K_TRACE][0]><<<grid, block, 0, s>>>(a); break;
-      case 1: k_trace_tile<NS, MIX, kMinBlocks[K_TRACE][1]><<<grid, block, 0, s>>>(a); break;
-      case 2: k_trace_tile<NS, MIX, kMinBlocks[K_TRACE][2]><<<grid, block, 0, s>>>(a); break;
+      case 0: return launch_kernel(k_trace_tile<NS, MIX, kMinBlocks[K_TRACE][0]>, grid, a, s);
+      case 1: return launch_kernel(k_trace_tile<NS, MIX, kMinBlocks[K_TRACE][1]>, grid, a, s);
+      case 2: return launch_kernel(k_trace_tile<NS, MIX, kMinBlocks[K_TRACE][2]>, grid, a, s);
       default: return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
   } else {
     return cudaErrorInvalidValue;  // the FP64 forms and large species counts trace per cell
   }
@@ -86,14 +82,14 @@ static cudaError_t launch_trace_tile(const pcg::StageArgs& a, const dim3& grid, 
 template <int NS, bool MIX, class R>
 static cudaError_t launch_t(int stage, const pcg::StageArgs& a, int64_t nblocks, int variant, cudaStream_t s) {
   if (nblocks <= 0) return cudaSuccess;
-  const dim3 grid((unsigned)nblocks), block(128);
-  if (stage == K_TRACE_TILE) return launch_trace_tile<NS, MIX, R>(a, grid, block, variant, s);
+  const unsigned grid = (unsigned)nblocks;
+  if (stage == K_TRACE_TILE) return launch_trace_tile<NS, MIX, R>(a, grid, variant, s);
   if (stage == K_SRCQ || (a.umeth && (stage == K_FLUX2 || stage == K_LOWBC || stage == K_CONSUP)))
-    return launch_special<NS, MIX, R>(stage, a, grid, block, s);
+    return launch_special<NS, MIX, R>(stage, a, grid, s);
   switch (variant) {
-    case 0: return launch_v<NS, MIX, R, 0>(stage, a, grid, block, s);
-    case 1: return launch_v<NS, MIX, R, 1>(stage, a, grid, block, s);
-    case 2: return launch_v<NS, MIX, R, 2>(stage, a, grid, block, s);
+    case 0: return launch_v<NS, MIX, R, 0>(stage, a, grid, s);
+    case 1: return launch_v<NS, MIX, R, 1>(stage, a, grid, s);
+    case 2: return launch_v<NS, MIX, R, 2>(stage, a, grid, s);
     default: return cudaErrorInvalidValue;
   }
 }

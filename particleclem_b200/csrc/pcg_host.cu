@@ -823,9 +823,26 @@ void bind_tables(Tables& T) {
   for (int s = 0; s < K_NKIND; ++s) T.segs[s] = reinterpret_cast<const pcg::Seg*>(base + reinterpret_cast<size_t>(T.segs[s]));
 }
 
+// The segment count of a launch, and the segments themselves where they fit its arguments.
+template <class A>
+void set_segs(A& a, const std::vector<pcg::Seg>& v) {
+  a.nseg = (int32_t)v.size();
+  if (v.size() <= size_t(pcg::kFewSegs)) std::copy(v.begin(), v.end(), a.few);
+}
+
+// The overlap of a launch of nblocks blocks with the launches before (after) and behind
+// (more) it, where those are the library's own in the same call. It saves the launch gap, a
+// few microseconds per launch, and costs each block about 0.3 us at its start (traces of
+// 17000 and 51000 blocks ran 3-5 % longer with it), so launches of many waves go without.
+constexpr int64_t kOverlapBlocks = 4096;
+int overlap_launch(int64_t nblocks, bool after, bool more) {
+  if (nblocks > kOverlapBlocks) return 0;
+  return (after ? pcg::kOverlapPrevious : 0) | (more ? pcg::kOverlapNext : 0);
+}
+
 // One launch of the kernel of `stage` over the segments of kind `segs` (launch variant var).
 int launch_segs(const Layout& L, const Tables& T, const pcg_hydro_params* p, int stage, int segs, int var,
-                const double* dt_dev, cudaStream_t s) {
+                const double* dt_dev, bool after, bool more, cudaStream_t s) {
   if (L.nblocks[segs] == 0) return PCG_OK;
   const bool single = p->precision_mode == PCG_PREC_MIXED;
   pcg::StageArgs a{};
@@ -833,13 +850,14 @@ int launch_segs(const Layout& L, const Tables& T, const pcg_hydro_params* p, int
   a.err = T.err;
   a.regions = T.regions;
   a.segs = T.segs[segs];
-  a.nseg = (int32_t)L.segs[segs].size();
+  set_segs(a, L.segs[segs]);
   a.ppm_type = p->ppm_type;
   a.plm_iorder = p->plm_iorder;
   a.use_flattening = p->use_flattening;
   a.use_hybrid_weno = p->use_hybrid_weno;
   a.weno_scheme = p->weno_scheme;
   a.umeth = L.umeth;
+  a.overlap = overlap_launch(L.nblocks[segs], after, more);
   a.difmag = p->difmag;
   a.dt_dev = dt_dev;
   cudaError_t e = (p->precision_mode == PCG_PREC_FP64)
@@ -850,21 +868,23 @@ int launch_segs(const Layout& L, const Tables& T, const pcg_hydro_params* p, int
 }
 
 int launch_kind(const Layout& L, const Tables& T, const pcg_hydro_params* p, int kind, const double* dt_dev,
-                cudaStream_t s) {
+                bool after, bool more, cudaStream_t s) {
   int var = kind < K_NSTAGE ? variant_of(p->precision_mode, L.ns, kind) : 0;
   if (var >= kTileVariant) {
     var -= kTileVariant;
     // the mixed form's tiled trace (variants 3-5), when every tensor map was encoded
     if (kind == K_TRACE && L.tile_trace && T.maps_ok) kind = K_TRACE_TILE;
   }
-  return launch_segs(L, T, p, kind, kind, var, dt_dev, s);
+  return launch_segs(L, T, p, kind, kind, var, dt_dev, after, more, s);
 }
 
+// after, more: the call has launches of its own before the first stage, behind the last.
 int launch_stages(const Layout& L, const Tables& T, const pcg_hydro_params* p, int first, int last,
-                  const double* dt_dev, cudaStream_t s) {
+                  const double* dt_dev, cudaStream_t s, bool after = false, bool more = false) {
   for (int st = first; st <= last; ++st) {
-    int rc = launch_kind(L, T, p, st, dt_dev, s);
-    if (rc == PCG_OK && st == K_FLUX2) rc = launch_kind(L, T, p, K_LOWBC, dt_dev, s);
+    const bool next = st < last || more;
+    int rc = launch_kind(L, T, p, st, dt_dev, after || st > first, next, s);
+    if (rc == PCG_OK && st == K_FLUX2) rc = launch_kind(L, T, p, K_LOWBC, dt_dev, true, next, s);
     if (rc) return rc;
   }
   return PCG_OK;
@@ -1309,7 +1329,7 @@ int pcg_srctoprim(const pcg_hydro_params* prm, const int32_t lo[3], const int32_
     bind_tables(T);
     pcg_hydro_params p = *prm;
     p.precision_mode = PCG_PREC_FP64;  // FP64 in every form, reference operation order
-    rc = launch_kind(L, T, &p, K_SRCQ, nullptr, s);
+    rc = launch_kind(L, T, &p, K_SRCQ, nullptr, false, false, s);
   } else {
     rc = fail(PCG_ECUDA, "table upload: %s", cudaGetErrorString(e));
   }
@@ -1423,16 +1443,18 @@ int pcg_step_boxes(const pcg_hydro_params* prm, int32_t nbox, const pcg_box* box
     f.nfill = nbox;
     f.ng = 4;
     f.ncomp = nv;
+    f.overlap = overlap_launch(fill_blocks, false, true);
     e = pcg_strict::launch_aux(AUX_FILL_BOXES, prm->nspec, f, fill_blocks, s);
     if (e != cudaSuccess) rc = fail(PCG_ECUDA, "ghost fill: %s", cudaGetErrorString(e));
   }
-  if (!rc) rc = launch_stages(L, T2, prm, K_CTOPRIM, K_FLUX2, nullptr, s);
+  if (!rc) rc = launch_stages(L, T2, prm, K_CTOPRIM, K_FLUX2, nullptr, s, fill_ghosts != 0, true);
   if (!rc) {
     pcg::StageArgs a{};
     a.regions = T2.regions;
     a.segs = T2.segs[K_CONSUP];
-    a.nseg = (int32_t)L.segs[K_CONSUP].size();
+    set_segs(a, L.segs[K_CONSUP]);
     a.partial = partial;
+    a.overlap = overlap_launch(L.nblocks[K_CONSUP], true, true);
     const int v = variant_of(prm->precision_mode, prm->nspec, K_CONSUP);
     e = strict ? pcg_strict::launch_advance(prm->nspec, a, L.nblocks[K_CONSUP], v, s)
                : pcg_fast::launch_advance(prm->nspec, a, L.nblocks[K_CONSUP], v, s);
@@ -1442,6 +1464,7 @@ int pcg_step_boxes(const pcg_hydro_params* prm, int32_t nbox, const pcg_box* box
       r.partial = partial;
       r.cfl = cfl;
       r.dt_boxes = dt_next;
+      r.overlap = overlap_launch(nbox, true, false);
       e = pcg_strict::launch_aux(AUX_ESTDT_BOXES, prm->nspec, r, nbox, s);
     }
     if (e != cudaSuccess) rc = fail(PCG_ECUDA, "step tail: %s", cudaGetErrorString(e));
@@ -1502,12 +1525,14 @@ int pcg_estdt(int32_t nspec, int32_t nbox, const pcg_box* boxes, double cfl, dou
     pcg::AuxArgs a{};
     a.boxes = reinterpret_cast<const pcg::AuxBox*>(dev);
     a.segs = reinterpret_cast<const pcg::Seg*>(dev + b1);
-    a.nseg = (int32_t)segs.size();
+    set_segs(a, segs);
     a.partial = reinterpret_cast<double*>(dev + b1 + b2);
     a.npartial = nblocks;
     a.cfl = cfl;
     a.dt_out = dt_out;
+    a.overlap = overlap_launch(nblocks, false, true);
     e = pcg_strict::launch_aux(AUX_ESTDT, nspec, a, nblocks, s);
+    a.overlap = pcg::kOverlapPrevious;
     if (e == cudaSuccess) e = pcg_strict::launch_aux(AUX_ESTDT_FINAL, nspec, a, 1, s);
   }
   if (e != cudaSuccess) rc = fail(PCG_ECUDA, "estdt: %s", cudaGetErrorString(e));
@@ -1552,7 +1577,7 @@ int pcg_update_state(int32_t nspec, int32_t nbox, const pcg_box* boxes, const pc
     pcg::AuxArgs a{};
     a.boxes = reinterpret_cast<const pcg::AuxBox*>(dev);
     a.segs = reinterpret_cast<const pcg::Seg*>(dev + b1);
-    a.nseg = (int32_t)segs.size();
+    set_segs(a, segs);
     a.dt_in = dt;
     e = pcg_strict::launch_aux(AUX_UPDATE, nspec, a, nblocks, s);
   }
@@ -1744,13 +1769,15 @@ int pcg_plan_estdt(pcg_plan* P, double cfl, double* dt_dev, pcg_stream_t stream)
   pcg::AuxArgs a{};
   a.boxes = P->d_aux;
   a.segs = P->d_aux_segs;
-  a.nseg = (int32_t)P->aux_segs.size();
+  set_segs(a, P->aux_segs);
   a.partial = P->d_partial;
   a.npartial = P->aux_blocks;
   a.cfl = cfl;
   a.dt_out = dt_dev;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  a.overlap = overlap_launch(P->aux_blocks, false, true);
   cudaError_t e = pcg_strict::launch_aux(AUX_ESTDT, P->prm.nspec, a, P->aux_blocks, s);
+  a.overlap = pcg::kOverlapPrevious;
   if (e == cudaSuccess) e = pcg_strict::launch_aux(AUX_ESTDT_FINAL, P->prm.nspec, a, 1, s);
   return e == cudaSuccess ? PCG_OK : fail(PCG_ECUDA, "estdt: %s", cudaGetErrorString(e));
 }
@@ -1762,7 +1789,7 @@ int pcg_plan_update(pcg_plan* P, const double* dt_dev, pcg_stream_t stream) {
   pcg::AuxArgs a{};
   a.boxes = P->d_aux;
   a.segs = P->d_aux_segs;
-  a.nseg = (int32_t)P->aux_segs.size();
+  set_segs(a, P->aux_segs);
   a.dt_in = dt_dev;
   cudaError_t e = pcg_strict::launch_aux(AUX_UPDATE, P->prm.nspec, a, P->aux_blocks, reinterpret_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? PCG_OK : fail(PCG_ECUDA, "update: %s", cudaGetErrorString(e));
@@ -1773,14 +1800,15 @@ int pcg_plan_advance(pcg_plan* P, double cfl, const double* dt_dev, double* dt_n
   int rc = ensure_eos(P->prm.nspec);
   if (rc) return rc;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if ((rc = launch_stages(P->L, P->T, &P->prm, K_CTOPRIM, K_FLUX2, dt_dev, s))) return rc;
+  if ((rc = launch_stages(P->L, P->T, &P->prm, K_CTOPRIM, K_FLUX2, dt_dev, s, false, true))) return rc;
   pcg::StageArgs a{};
   a.regions = P->T.regions;
   a.segs = P->T.segs[K_CONSUP];
-  a.nseg = (int32_t)P->L.segs[K_CONSUP].size();
+  set_segs(a, P->L.segs[K_CONSUP]);
   a.dt_dev = dt_dev;
   a.partial = P->d_partial;
   const int64_t nb = P->L.nblocks[K_CONSUP];
+  a.overlap = overlap_launch(nb, true, true);
   const int v = variant_of(P->prm.precision_mode, P->prm.nspec, K_CONSUP);
   cudaError_t e = (P->prm.precision_mode == PCG_PREC_FP64) ? pcg_strict::launch_advance(P->prm.nspec, a, nb, v, s)
                                                            : pcg_fast::launch_advance(P->prm.nspec, a, nb, v, s);
@@ -1790,6 +1818,7 @@ int pcg_plan_advance(pcg_plan* P, double cfl, const double* dt_dev, double* dt_n
     f.npartial = nb;
     f.cfl = cfl;
     f.dt_out = dt_next;
+    f.overlap = pcg::kOverlapPrevious;
     e = pcg_strict::launch_aux(AUX_ESTDT_FINAL, P->prm.nspec, f, 1, s);
   }
   return e == cudaSuccess ? PCG_OK : fail(PCG_ECUDA, "advance: %s", cudaGetErrorString(e));

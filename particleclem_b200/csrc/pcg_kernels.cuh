@@ -57,17 +57,47 @@ __device__ __forceinline__ double dt_of(const pcg::StageArgs& a, const pcg::Regi
   return a.dt_dev ? *a.dt_dev : rg.dt_ptr ? *rg.dt_ptr : rg.dt;
 }
 
+// Successive launches of one call may overlap (programmatic dependent launch, StageArgs::
+// overlap): a kernel with kOverlapNext lets the next one's blocks start as soon as its own
+// have all started; one with kOverlapPrevious waits, before it touches anything an earlier
+// launch writes, until the launch before it has completed and its results are visible. Every
+// thread passes here first, also those that then leave, so a kernel is complete only after all
+// earlier ones are. What
+// overlaps is the launch itself, the start of the blocks in the slots the last blocks of the
+// previous kernel leave, and the segment lookup below.
+__device__ __forceinline__ void await_previous(int overlap) {
+  if (overlap & pcg::kOverlapNext) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (overlap & pcg::kOverlapPrevious) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// The segment of this block. A launch of few segments carries them in its arguments, so its
+// blocks know their work without a load, before the wait; longer tables are searched in
+// memory after it.
+__device__ __forceinline__ pcg::Seg find_seg(const pcg::Seg* few, const pcg::Seg* segs, int nseg, int overlap) {
+  const int blk = blockIdx.x;
+  if (nseg <= pcg::kFewSegs) {
+    int s = 0;
+#pragma unroll
+    for (int m = 1; m < pcg::kFewSegs; ++m)
+      if (m < nseg && (int)few[m].blk0 <= blk) s = m;
+    const pcg::Seg sg = few[s];
+    await_previous(overlap);
+    return sg;
+  }
+  await_previous(overlap);
+  int lo = 0, hi = nseg - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (segs[mid].blk0 <= blk) lo = mid; else hi = mid - 1;
+  }
+  return segs[lo];
+}
+
 // Segment counts and block numbers stay below 2^31 (the host checks the launch sizes),
 // so the thread's position is formed with 32-bit (unsigned) division.
 __device__ __forceinline__ bool item_of(const pcg::StageArgs& a, Item& it) {
-  const int blk = blockIdx.x;
-  int lo = 0, hi = a.nseg - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (a.segs[mid].blk0 <= blk) lo = mid; else hi = mid - 1;
-  }
-  const pcg::Seg& s = a.segs[lo];
-  const unsigned local = unsigned(blk - (int)s.blk0) * blockDim.x + threadIdx.x;
+  const pcg::Seg s = find_seg(a.few, a.segs, a.nseg, a.overlap);
+  const unsigned local = unsigned(int(blockIdx.x) - (int)s.blk0) * blockDim.x + threadIdx.x;
   if (local >= (unsigned)s.count) return false;
   const unsigned n0 = s.n[0], n1 = s.n[1];
   const unsigned t = local / n0;
@@ -80,15 +110,10 @@ __device__ __forceinline__ bool item_of(const pcg::StageArgs& a, Item& it) {
 }
 
 // The segment of this block and the block's index within it (tiled stages).
-__device__ __forceinline__ const pcg::Seg& seg_of(const pcg::StageArgs& a, int& local_block) {
-  const int blk = blockIdx.x;
-  int lo = 0, hi = a.nseg - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (a.segs[mid].blk0 <= blk) lo = mid; else hi = mid - 1;
-  }
-  local_block = blk - (int)a.segs[lo].blk0;
-  return a.segs[lo];
+__device__ __forceinline__ pcg::Seg seg_of(const pcg::StageArgs& a, int& local_block) {
+  const pcg::Seg s = find_seg(a.few, a.segs, a.nseg, a.overlap);
+  local_block = int(blockIdx.x) - (int)s.blk0;
+  return s;
 }
 
 // A pointer positioned at one cell of a view: components n at p[n * ns].
@@ -150,7 +175,7 @@ __device__ __forceinline__ double p0_of(const pcg::Region& rg) {
 // ------------------------------------------------------------------ ctoprim
 // Source/PeleCUtilities.H:242-320 (pc_ctoprim), omega = rad = 0.
 template <int NS, bool MIX, int MINB>
-__global__ void __launch_bounds__(128, MINB) k_ctoprim(pcg::StageArgs a) {
+__global__ void __launch_bounds__(128, MINB) k_ctoprim(const __grid_constant__ pcg::StageArgs a) {
   Item it;
   if (!item_of(a, it)) return;
   const pcg::Region& rg = *it.rg;
@@ -296,7 +321,7 @@ __device__ __forceinline__ void prep_cell(const pcg::StageArgs& a, const pcg::Re
 // flattening is evaluated in the compute type R: FP64 in the FP64 forms, FP32 in the
 // mixed form (the primitive values rounded to FP32; it departs from 1 only at shocks).
 template <int NS, bool MIX, bool EXACT, class R>
-__global__ void __launch_bounds__(128) k_prep(pcg::StageArgs a) {
+__global__ void __launch_bounds__(128) k_prep(const __grid_constant__ pcg::StageArgs a) {
   Item it;
   if (!item_of(a, it)) return;
   const pcg::Region& rg = *it.rg;
@@ -648,7 +673,7 @@ __device__ __forceinline__ void trace_cell(const pcg::StageArgs& a, const pcg::R
 }
 
 template <int NS, bool MIX, bool EXACT, class R, int MINB>
-__global__ void __launch_bounds__(128, MINB) k_trace(pcg::StageArgs a) {
+__global__ void __launch_bounds__(128, MINB) k_trace(const __grid_constant__ pcg::StageArgs a) {
   Item it;
   if (!item_of(a, it)) return;
   switch (it.variant) {
@@ -813,7 +838,7 @@ __device__ __forceinline__ void trace_tile(const pcg::StageArgs& a, const pcg::S
 }
 
 template <int NS, bool MIX, int MINB>
-__global__ void __launch_bounds__(128, MINB) k_trace_tile(pcg::StageArgs a) {
+__global__ void __launch_bounds__(128, MINB) k_trace_tile(const __grid_constant__ pcg::StageArgs a) {
   constexpr int kBoxMax = pcg::trace_box_cells(1) > pcg::trace_box_cells(2) ? pcg::trace_box_cells(1)
                                                                              : pcg::trace_box_cells(2);
   static_assert(pcg::trace_box_cells(0) <= kBoxMax, "tile buffer");
@@ -826,7 +851,7 @@ __global__ void __launch_bounds__(128, MINB) k_trace_tile(pcg::StageArgs a) {
   __shared__ __align__(8) uint64_t bar;
   static_assert(sizeof(tile) + sizeof(dsv) + sizeof(edg) + 8 <= 48 * 1024, "tile shared memory");
   int t;
-  const pcg::Seg& sg = seg_of(a, t);
+  const pcg::Seg sg = seg_of(a, t);
   if (sg.variant < 3) {  // a strip: one cell per thread (the block's segment is uniform)
     const unsigned local = unsigned(t) * blockDim.x + threadIdx.x;
     if (local >= (unsigned)sg.count) return;
@@ -853,7 +878,7 @@ __global__ void __launch_bounds__(128, MINB) k_trace_tile(pcg::StageArgs a) {
 // The PPM trace with hybrid-WENO edge values (use_hybrid_weno): its own kernel, so that
 // the WENO code does not weigh on the registers of the plain trace.
 template <int NS, bool MIX, bool EXACT, class R>
-__global__ void __launch_bounds__(128) k_trace_weno(pcg::StageArgs a) {
+__global__ void __launch_bounds__(128) k_trace_weno(const __grid_constant__ pcg::StageArgs a) {
   Item it;
   if (!item_of(a, it)) return;
   switch (it.variant) {
@@ -906,7 +931,7 @@ __device__ __forceinline__ void flux0_face(const pcg::Region& rg, int i, int j, 
 }
 
 template <int NS, bool MIX, bool EXACT, class R, int MINB>
-__global__ void __launch_bounds__(128, MINB) k_flux0(pcg::StageArgs a) {
+__global__ void __launch_bounds__(128, MINB) k_flux0(const __grid_constant__ pcg::StageArgs a) {
   Item it;
   if (!item_of(a, it)) return;
   switch (it.variant) {
@@ -1219,11 +1244,11 @@ __device__ __forceinline__ void flux1_face(const pcg::StageArgs& a, const pcg::R
 }
 
 template <int NS, bool MIX, bool EXACT, class R, int MINB>
-__global__ void __launch_bounds__(128, MINB) k_flux1(pcg::StageArgs a) {
+__global__ void __launch_bounds__(128, MINB) k_flux1(const __grid_constant__ pcg::StageArgs a) {
   if constexpr (pcg::flux1_shared(sizeof(R))) {
     __shared__ R kcarry[2 * ncorr1<NS>() * 128];
     int t;
-    const pcg::Seg& sg = seg_of(a, t);
+    const pcg::Seg sg = seg_of(a, t);
     switch (sg.variant) {
       case 0: flux1_x<NS, MIX, EXACT, R>(a, sg, t, kcarry); break;
       case 1: flux1_march<NS, MIX, EXACT, 1, R>(a, sg, t, kcarry); break;
@@ -1617,10 +1642,10 @@ __device__ __forceinline__ void flux2_march(const pcg::StageArgs& a, const pcg::
 }
 
 template <int NS, bool MIX, bool EXACT, class R, int MINB, bool UMETH = false>
-__global__ void __launch_bounds__(128, MINB) k_flux2(pcg::StageArgs a) {
+__global__ void __launch_bounds__(128, MINB) k_flux2(const __grid_constant__ pcg::StageArgs a) {
   __shared__ R kcarry[flux2_slots<NS, R>() * ncorr<NS>() * 128];
   int t;
-  const pcg::Seg& sg = seg_of(a, t);
+  const pcg::Seg sg = seg_of(a, t);
   switch (sg.variant) {
     case 0: flux2_x<NS, MIX, EXACT, R, UMETH>(a, sg, t, kcarry); break;
     case 1: flux2_march<NS, MIX, EXACT, 1, R, UMETH>(a, sg, t, kcarry); break;
@@ -1651,7 +1676,7 @@ __device__ __forceinline__ void lowbc_face(const pcg::StageArgs& a, const pcg::R
 }
 
 template <int NS, bool MIX, bool EXACT, class R, bool UMETH = false>
-__global__ void __launch_bounds__(128) k_lowbc(pcg::StageArgs a) {
+__global__ void __launch_bounds__(128) k_lowbc(const __grid_constant__ pcg::StageArgs a) {
   Item it;
   if (!item_of(a, it)) return;
   switch (it.variant) {
@@ -1664,7 +1689,7 @@ __global__ void __launch_bounds__(128) k_lowbc(pcg::StageArgs a) {
 // Source/Godunov.H:1033-1060 (pc_pdivu) from pc_umeth_3D's own face states (the caller's
 // NGDNV-component qec arrays of pcg_umeth), in the reference's expression order.
 template <int NS>
-__global__ void __launch_bounds__(128) k_pdivu(pcg::StageArgs a) {
+__global__ void __launch_bounds__(128) k_pdivu(const __grid_constant__ pcg::StageArgs a) {
   Item it;
   if (!item_of(a, it)) return;
   const pcg::Region& rg = *it.rg;
@@ -1688,7 +1713,7 @@ __global__ void __launch_bounds__(128) k_pdivu(pcg::StageArgs a) {
 // the primitive-variable sources srcQ from the conserved sources src and q, qaux. Only the
 // components the reference writes are written (not QGAME, QTEMP).
 template <int NS>
-__global__ void __launch_bounds__(128) k_srctoprim(pcg::StageArgs a) {
+__global__ void __launch_bounds__(128) k_srctoprim(const __grid_constant__ pcg::StageArgs a) {
   Item it;
   if (!item_of(a, it)) return;
   const pcg::Region& rg = *it.rg;
@@ -1795,7 +1820,7 @@ __device__ __forceinline__ void consup_cell(const pcg::Region& rg, int i, int j,
 }
 
 template <int NS, bool MIX>
-__global__ void __launch_bounds__(128) k_consup(pcg::StageArgs a) {
+__global__ void __launch_bounds__(128) k_consup(const __grid_constant__ pcg::StageArgs a) {
   Item it;
   if (!item_of(a, it)) return;
   const pcg::Region& rg = *it.rg;

@@ -163,6 +163,13 @@ struct Seg {
   int64_t blk0;  // first block of this segment within the launch
 };
 
+// Launches of up to this many segments (one region: three directions) carry them by value
+// in their arguments.
+constexpr int kFewSegs = 4;
+// StageArgs/AuxArgs::overlap (see await_previous): this launch may start while the one before
+// it in the call runs; the next launch may start while this one runs.
+enum { kOverlapPrevious = 1, kOverlapNext = 2 };
+
 struct StageArgs {
   const Region* regions;
   const Seg* segs;
@@ -173,11 +180,13 @@ struct StageArgs {
   int32_t use_hybrid_weno;
   int32_t weno_scheme;
   int32_t umeth;  // the call is pcg_umeth (see Region::umeth)
+  int32_t overlap;  // kOverlap* bits
   double difmag;
   const double* dt_dev;  // nullptr: each region's dt
   double* partial;       // fused step tail: one timestep minimum per block
   const void* tmaps;     // TMA-staged trace: 3 tensor maps (x, y, z boxes) per region
   int32_t* err;          // device error word: bit 0 set when a bounded TMA wait gave up
+  Seg few[kFewSegs];     // the segments when nseg <= kFewSegs
 };
 // The tiles of the TMA-staged trace, one per block of 128 threads: 32 cells along x by 4
 // along y (x and y traces) or along z (z trace), so that the 4 warps of a block are the
@@ -232,10 +241,11 @@ struct AuxArgs {
   int32_t periodic;     // ghost fill: bit d set when direction d is periodic
   const FillBox* fills; // batched ghost fill
   int32_t nfill;
-  int32_t pad;
+  int32_t overlap;      // kOverlap* bits
   View dst;               // device box copy: destination (state is the source)
   const pcg::Seg* bsegs;  // per-box timestep: the advance segments of each region
   double* dt_boxes;       // per-box timestep result (device, one per region)
+  Seg few[kFewSegs];      // the segments when nseg <= kFewSegs
 };
 
 }  // namespace pcg
