@@ -407,6 +407,7 @@ struct BoxIn {
 
 struct Layout {
   bool oversize = false;  // a workspace array would span 2^31 elements or more
+  int march = pcg::FACE_MARCH;  // faces per thread of the marching stages (face_march)
   bool tile_trace = false;  // the mixed form's trace runs as TMA-staged tiles (K_TRACE_TILE)
   int ns = 1;
   int umeth = 0;  // the plan is a pcg_umeth call
@@ -443,10 +444,11 @@ void add_seg(Layout& L, int stage, int region, int variant, const IBox& b) {
   s.variant = variant;
   for (int d = 0; d < 3; ++d) { s.lo[d] = b.lo[d]; s.n[d] = (int)b.n(d); }
   s.count = b.cells();
+  s.march = L.march;
   s.blk0 = L.nblocks[stage];
   L.segs[stage].push_back(s);
   const bool tiled = stage == K_FLUX2 || (stage == K_FLUX1 && pcg::flux1_shared(L.esz));
-  L.nblocks[stage] += tiled ? pcg::face_tiles(variant, s.n) : (s.count + kThreads - 1) / kThreads;
+  L.nblocks[stage] += tiled ? pcg::face_tiles(variant, s.n, s.march) : (s.count + kThreads - 1) / kThreads;
 }
 
 // Work order within a launch. Blocks start roughly in launch order, so the order of the
@@ -563,9 +565,26 @@ void add_trace_tiles(Layout& L, int region, int d, const IBox& g1) {
     sg.n[e] = (int)(core[e] / tn[e]);
   }
   sg.count = int64_t(sg.n[0]) * sg.n[1] * sg.n[2];
+  sg.march = L.march;
   sg.blk0 = L.nblocks[K_TRACE_TILE];
   L.segs[K_TRACE_TILE].push_back(sg);
   L.nblocks[K_TRACE_TILE] += sg.count;
+}
+
+// Faces each thread of a marching stage takes in turn along y or z. A march shares the
+// correction of the cell between two faces (4 faces need 5 corrections, 4 single faces 8),
+// but its faces come one after the other, and a small call leaves the chip idle meanwhile:
+// then shorter marches on more threads finish sooner.
+#ifndef PCG_MARCH_CELLS1
+#define PCG_MARCH_CELLS1 60000
+#endif
+#ifndef PCG_MARCH_CELLS2
+#define PCG_MARCH_CELLS2 120000
+#endif
+int face_march(const std::vector<BoxIn>& boxes) {
+  int64_t cells = 0;
+  for (const BoxIn& b : boxes) cells += b.bx.cells();
+  return cells <= PCG_MARCH_CELLS1 ? 1 : cells <= PCG_MARCH_CELLS2 ? 2 : pcg::FACE_MARCH;
 }
 
 void build_layout(Layout& L, const std::vector<BoxIn>& boxes, const pcg_hydro_params* prm) {
@@ -575,6 +594,7 @@ void build_layout(Layout& L, const std::vector<BoxIn>& boxes, const pcg_hydro_pa
   const int qf_grow = (prm->use_hybrid_weno && prm->ppm_type == 1 && prm->weno_scheme == 2) ? 4 : 3;
   L.ns = ns;
   L.esz = single ? 4 : 8;
+  L.march = face_march(boxes);
   // the mixed form traces from TMA-staged shared-memory tiles of its FP32 primitive copy
   // (PPM without hybrid WENO, and PLM)
   L.tile_trace = single && !prm->use_hybrid_weno && pcg::trace_tile_species(ns);

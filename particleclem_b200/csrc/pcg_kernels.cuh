@@ -942,18 +942,18 @@ __global__ void __launch_bounds__(128, MINB) k_flux0(const __grid_constant__ pcg
 }
 
 // The march of one thread of a y- or z-face stage (k_flux1, k_flux2): threads in linear
-// order over i (fastest), the row axis and the chunks of pcg::FACE_MARCH faces along D.
+// order over i (fastest), the row axis and the chunks of sg.march faces along D.
 template <int D>
 __device__ __forceinline__ bool march_of(const pcg::Seg& sg, int t, int& i, int& r, int& m0, int& m1) {
   constexpr int RA = (D == 1) ? 2 : 1;
   const unsigned local = unsigned(t) * blockDim.x + threadIdx.x;
-  if (local >= (unsigned)pcg::face_threads(D, sg.n)) return false;
+  if (local >= (unsigned)pcg::face_threads(D, sg.n, sg.march)) return false;
   const unsigned n0 = sg.n[0], nr = sg.n[RA];
   const unsigned q = local / n0;
   i = sg.lo[0] + (int)(local - q * n0);
   r = sg.lo[RA] + (int)(q % nr);
-  m0 = sg.lo[D] + (int)(q / nr) * pcg::FACE_MARCH;
-  m1 = min(m0 + pcg::FACE_MARCH, sg.lo[D] + sg.n[D]);
+  m0 = sg.lo[D] + (int)(q / nr) * sg.march;
+  m1 = min(m0 + sg.march, sg.lo[D] + sg.n[D]);
   return true;
 }
 
@@ -1165,7 +1165,7 @@ __device__ __forceinline__ void flux1_x(const pcg::StageArgs& a, const pcg::Seg&
   flux1_x_pair<NS, MIX, EXACT, 2, R>(a, rg, active, own_right, i, j, k, p0, kx + ncorr1<NS>() * 128);
 }
 
-// y- and z-faces: each thread marches pcg::FACE_MARCH faces along D (threads in linear
+// y- and z-faces: each thread marches sg.march faces along D (threads in linear
 // order over i, the row axis and the march chunks). Per partner O the correction of
 // the cell behind the face waits in the thread's shared-memory slot (component-major).
 template <int NS, bool MIX, bool EXACT, int D, int O, class R>
@@ -1520,7 +1520,7 @@ __device__ __forceinline__ void flux2_face(const pcg::StageArgs& a, const pcg::R
 //  * x-faces, one per thread in linear order: the correction right of a face comes from
 //    the next lane's shared-memory slot (the last lane of a warp and the last face of a
 //    row form it themselves);
-//  * y- and z-faces: each thread marches pcg::FACE_MARCH faces along D, carrying the
+//  * y- and z-faces: each thread marches sg.march faces along D, carrying the
 //    correction of the cell behind the face.
 // Block counts per segment are pcg::face_tiles on the host.
 template <int NS, bool MIX, bool EXACT, class R>

@@ -143,13 +143,16 @@ struct Region {
 // [lo, lo + n).
 // Blocks (of 128 threads) of the stages that share a cell's transverse correction
 // between its two faces (k_flux1, k_flux2): x-faces one face per thread; y- and
-// z-faces one thread per FACE_MARCH consecutive faces along their direction.
+// z-faces one thread per `march` consecutive faces along their direction (Seg::march, up to
+// FACE_MARCH; the host's face_march picks it per call).
 constexpr int FACE_MARCH = 4;
-PCG_HD constexpr int64_t face_threads(int d, const int32_t n[3]) {
+PCG_HD constexpr int64_t face_threads(int d, const int32_t n[3], int march) {
   return d == 0 ? int64_t(n[0]) * n[1] * n[2]
-                : int64_t(n[0]) * n[d == 1 ? 2 : 1] * ((n[d] + FACE_MARCH - 1) / FACE_MARCH);
+                : int64_t(n[0]) * n[d == 1 ? 2 : 1] * ((n[d] + march - 1) / march);
 }
-PCG_HD constexpr int64_t face_tiles(int d, const int32_t n[3]) { return (face_threads(d, n) + 127) / 128; }
+PCG_HD constexpr int64_t face_tiles(int d, const int32_t n[3], int march) {
+  return (face_threads(d, n, march) + 127) / 128;
+}
 // k_flux1 shares corrections in the FP32 form only (element size of the compute type);
 // the FP64 forms run one face per thread.
 PCG_HD constexpr bool flux1_shared(size_t esz) { return esz == 4; }
@@ -159,6 +162,8 @@ struct Seg {
   int32_t variant;
   int32_t lo[3];
   int32_t n[3];
+  int32_t march;  // faces per thread along y and z in the stages that march
+  int32_t pad;
   int64_t count;
   int64_t blk0;  // first block of this segment within the launch
 };
