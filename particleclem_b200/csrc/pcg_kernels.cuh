@@ -1067,13 +1067,21 @@ __device__ __forceinline__ void transdo_apply(const R* qn, const KF& K, R p0, R*
   out[pcg::TR_P] = dmax(pnew, pfloor(Lim<R>::very_small(), p0));
 }
 
+// Both transverse partners O of a face run through one loop body, O a runtime value: with a
+// copy per partner, direction and temperature range the kernel outgrows the instruction
+// caches (FP64 reference order, 9 species: 4.6 of its 17 stall cycles per instruction were
+// instruction fetch). 128^3 flame level, one body against two copies: FP64 reference order
+// 2.23 / 3.07 ms, mixed 0.654 / 0.685 ms; the FP64 FMA form's body is small enough for two
+// (96^3: 0.661 / 0.613 ms).
+template <bool EXACT, class R> constexpr int flux1_copies() { return !EXACT && sizeof(R) == 8 ? 2 : 1; }
+
 // The O-correction of the cell (i, j, k): the first O-fluxes on its two O-faces and
 // its gamma_c.
-template <int NS, int O, class R>
-__device__ __forceinline__ void flux1_corr(const pcg::Region& rg, int i, int j, int k, R cdt, R p0, R* K) {
-  const B4<const R> fov = b4<const R>(rg.fi[O]);
+template <int NS, class R>
+__device__ __forceinline__ void flux1_corr(const pcg::Region& rg, int o, int i, int j, int k, R cdt, R p0, R* K) {
+  const B4<const R> fov = b4<const R>(rg.fi[o]);
   const R c = R(v4<const double>(rg.qa)(i, j, k, pcg::QGAMC));
-  transdo_corr<NS, R>(at(fov, i, j, k), at_up(fov, i, j, k, O), cdt, c, p0, K);
+  transdo_corr<NS, R>(at(fov, i, j, k), at_up(fov, i, j, k, o), cdt, c, p0, K);
 }
 
 // The (D|O) flux at the D-face (i, j, k) from the left and right O-corrections
@@ -1090,33 +1098,25 @@ __device__ __forceinline__ void flux1_state(const pcg::Region& rg, int i, int j,
 }
 
 // The O-correction of the cell (i, j, k), formed on demand.
-template <int NS, int O, class R>
-__device__ __forceinline__ TransdoCorr<NS, R> flux1_corr_fn(const pcg::Region& rg, int i, int j, int k, R cdt, R p0) {
-  const B4<const R> fov = b4<const R>(rg.fi[O]);
-  return TransdoCorr<NS, R>{at(fov, i, j, k), at_up(fov, i, j, k, O), cdt,
+template <int NS, class R>
+__device__ __forceinline__ TransdoCorr<NS, R> flux1_corr_fn(const pcg::Region& rg, int o, int i, int j, int k, R cdt,
+                                                            R p0) {
+  const B4<const R> fov = b4<const R>(rg.fi[o]);
+  return TransdoCorr<NS, R>{at(fov, i, j, k), at_up(fov, i, j, k, o), cdt,
                             R(v4<const double>(rg.qa)(i, j, k, pcg::QGAMC)), p0};
 }
 
-template <int NS, bool MIX, bool EXACT, int D, int O, class R>
-__device__ __forceinline__ void flux1_riemann(const pcg::Region& rg, int i, int j, int k, const R* ql, const R* qr,
-                                              R p0) {
+template <int NS, bool MIX, bool EXACT, int D, class R>
+__device__ __forceinline__ void flux1_riemann(const pcg::Region& rg, int o, int i, int j, int k, const R* ql,
+                                              const R* qr, R p0) {
   R fl[pcg::nvar(NS)], gun, gpres;
   face_flux<NS, MIX, EXACT, D, R>(rg, i, j, k, ql, qr, p0, fl, gun, gpres);
-  store_tflux<NS, R>(at(b4<R>(rg.fdo[D][O]), i, j, k), fl, gun, gpres);
-}
-
-template <int NS, bool MIX, bool EXACT, int D, int O, class R>
-__device__ __forceinline__ void flux1_solve(const pcg::Region& rg, int i, int j, int k, const R* Kl, const R* Kr,
-                                            R p0) {
-  R ql[pcg::nt_comps(NS)], qr[pcg::nt_comps(NS)];
-  flux1_state<NS, EXACT, D, 0, R>(rg, i, j, k, Kl, p0, ql);
-  flux1_state<NS, EXACT, D, 1, R>(rg, i, j, k, Kr, p0, qr);
-  flux1_riemann<NS, MIX, EXACT, D, O, R>(rg, i, j, k, ql, qr, p0);
+  store_tflux<NS, R>(at(b4<R>(rg.fdo[D][o]), i, j, k), fl, gun, gpres);
 }
 
 template <int NS, class R>
-__device__ __forceinline__ R flux1_cdt(const pcg::StageArgs& a, const pcg::Region& rg, int O) {
-  return R(1.0 / 3.0 * dt_of(a, rg) / rg.dx[O]);
+__device__ __forceinline__ R flux1_cdt(const pcg::StageArgs& a, const pcg::Region& rg, int o) {
+  return R(1.0 / 3.0 * dt_of(a, rg) / rg.dx[o]);
 }
 
 // x-faces, one face per thread in linear order (i fastest): each lane forms the
@@ -1124,31 +1124,6 @@ __device__ __forceinline__ R flux1_cdt(const pcg::StageArgs& a, const pcg::Regio
 // lane's shared-memory slot, which holds that cell whenever it is in the same row; the
 // last lane of a warp and the last face of a row form it themselves. The (0|O) flux
 // exists where the face's O index lies in the box.
-template <int NS, bool MIX, bool EXACT, int O, class R>
-__device__ __forceinline__ void flux1_x_pair(const pcg::StageArgs& a, const pcg::Region& rg, bool active, bool own_right,
-                                             int i, int j, int k, R p0, R* kx) {
-  const int c[3] = {i, j, k};
-  const bool has = active && c[O] >= rg.lo[O] && c[O] <= rg.hi[O];
-  const R cdt = flux1_cdt<NS, R>(a, rg, O);
-  R* mine = kx + threadIdx.x;
-  R K[ncorr1<NS>()];
-  if (has) {
-    flux1_corr<NS, O, R>(rg, i - 1, j, k, cdt, p0, K);
-#pragma unroll
-    for (int n = 0; n < ncorr1<NS>(); ++n) mine[n * 128] = K[n];
-  }
-  __syncwarp();
-  if (!has) return;
-  R Kr[ncorr1<NS>()];
-  if (own_right) {
-    flux1_corr<NS, O, R>(rg, i, j, k, cdt, p0, Kr);
-  } else {
-#pragma unroll
-    for (int n = 0; n < ncorr1<NS>(); ++n) Kr[n] = mine[n * 128 + 1];
-  }
-  flux1_solve<NS, MIX, EXACT, 0, O, R>(rg, i, j, k, K, Kr, p0);
-}
-
 template <int NS, bool MIX, bool EXACT, class R>
 __device__ __forceinline__ void flux1_x(const pcg::StageArgs& a, const pcg::Seg& sg, int t, R* kx) {
   const pcg::Region& rg = a.regions[sg.region];
@@ -1161,29 +1136,36 @@ __device__ __forceinline__ void flux1_x(const pcg::StageArgs& a, const pcg::Seg&
   const int k = sg.lo[2] + (int)(q / n1);
   const bool own_right = (threadIdx.x & 31) == 31 || i == sg.lo[0] + sg.n[0] - 1;
   const R p0 = R(p0_of<NS, MIX, R>(rg));
-  flux1_x_pair<NS, MIX, EXACT, 1, R>(a, rg, active, own_right, i, j, k, p0, kx);
-  flux1_x_pair<NS, MIX, EXACT, 2, R>(a, rg, active, own_right, i, j, k, p0, kx + ncorr1<NS>() * 128);
+#pragma unroll(flux1_copies<EXACT, R>())
+  for (int o = 1; o < 3; ++o) {
+    const int c = o == 1 ? j : k;
+    const bool has = active && c >= rg.lo[o] && c <= rg.hi[o];
+    const R cdt = flux1_cdt<NS, R>(a, rg, o);
+    R* mine = kx + (o - 1) * ncorr1<NS>() * 128 + threadIdx.x;
+    R K[ncorr1<NS>()];
+    if (has) {
+      flux1_corr<NS, R>(rg, o, i - 1, j, k, cdt, p0, K);
+#pragma unroll
+      for (int n = 0; n < ncorr1<NS>(); ++n) mine[n * 128] = K[n];
+    }
+    __syncwarp();
+    if (!has) continue;
+    R ql[pcg::nt_comps(NS)], qr[pcg::nt_comps(NS)];
+    flux1_state<NS, EXACT, 0, 0, R>(rg, i, j, k, K, p0, ql);
+    if (own_right) {
+      flux1_corr<NS, R>(rg, o, i, j, k, cdt, p0, K);
+    } else {
+#pragma unroll
+      for (int n = 0; n < ncorr1<NS>(); ++n) K[n] = mine[n * 128 + 1];
+    }
+    flux1_state<NS, EXACT, 0, 1, R>(rg, i, j, k, K, p0, qr);
+    flux1_riemann<NS, MIX, EXACT, 0, R>(rg, o, i, j, k, ql, qr, p0);
+  }
 }
 
 // y- and z-faces: each thread marches sg.march faces along D (threads in linear
 // order over i, the row axis and the march chunks). Per partner O the correction of
 // the cell behind the face waits in the thread's shared-memory slot (component-major).
-template <int NS, bool MIX, bool EXACT, int D, int O, class R>
-__device__ __forceinline__ void flux1_march_pair(const pcg::Region& rg, int i, int r, int m, R cdt, R p0, R* slot) {
-  const int j = (D == 1) ? m : r, k = (D == 1) ? r : m;
-  R K[ncorr1<NS>()], qr[pcg::nt_comps(NS)], ql[pcg::nt_comps(NS)];
-  flux1_corr<NS, O, R>(rg, i, j, k, cdt, p0, K);
-  flux1_state<NS, EXACT, D, 1, R>(rg, i, j, k, K, p0, qr);
-#pragma unroll
-  for (int n = 0; n < ncorr1<NS>(); ++n) {
-    const R kl = slot[n * 128];
-    slot[n * 128] = K[n];
-    K[n] = kl;
-  }
-  flux1_state<NS, EXACT, D, 0, R>(rg, i, j, k, K, p0, ql);
-  flux1_riemann<NS, MIX, EXACT, D, O, R>(rg, i, j, k, ql, qr, p0);
-}
-
 template <int NS, bool MIX, bool EXACT, int D, class R>
 __device__ __forceinline__ void flux1_march(const pcg::StageArgs& a, const pcg::Seg& sg, int t, R* kcarry) {
   const pcg::Region& rg = a.regions[sg.region];
@@ -1194,23 +1176,28 @@ __device__ __forceinline__ void flux1_march(const pcg::StageArgs& a, const pcg::
   const bool has0 = i >= rg.lo[0] && i <= rg.hi[0];     // (D|0) exists
   const bool hasr = r >= rg.lo[RA] && r <= rg.hi[RA];  // (D|RA) exists
   const R cdt0 = flux1_cdt<NS, R>(a, rg, 0), cdtr = flux1_cdt<NS, R>(a, rg, RA);
-  R* s0 = kcarry + threadIdx.x;
-  R* sr = kcarry + ncorr1<NS>() * 128 + threadIdx.x;
-  R K[ncorr1<NS>()];
-  const int jb = (D == 1) ? m0 - 1 : r, kb = (D == 1) ? r : m0 - 1;
-  if (has0) {
-    flux1_corr<NS, 0, R>(rg, i, jb, kb, cdt0, p0, K);
+  // step m0 - 1 only fills the slots with the corrections of the cell behind the first face
+#pragma unroll 1
+  for (int m = m0 - 1; m < m1; ++m) {
+    const int j = (D == 1) ? m : r, k = (D == 1) ? r : m;
+#pragma unroll(flux1_copies<EXACT, R>())
+    for (int h = 0; h < 2; ++h) {
+      if (!(h == 0 ? has0 : hasr)) continue;
+      const int o = h == 0 ? 0 : RA;
+      R* slot = kcarry + h * ncorr1<NS>() * 128 + threadIdx.x;
+      R K[ncorr1<NS>()], qr[pcg::nt_comps(NS)], ql[pcg::nt_comps(NS)];
+      flux1_corr<NS, R>(rg, o, i, j, k, h == 0 ? cdt0 : cdtr, p0, K);
+      if (m >= m0) flux1_state<NS, EXACT, D, 1, R>(rg, i, j, k, K, p0, qr);
 #pragma unroll
-    for (int n = 0; n < ncorr1<NS>(); ++n) s0[n * 128] = K[n];
-  }
-  if (hasr) {
-    flux1_corr<NS, RA, R>(rg, i, jb, kb, cdtr, p0, K);
-#pragma unroll
-    for (int n = 0; n < ncorr1<NS>(); ++n) sr[n * 128] = K[n];
-  }
-  for (int m = m0; m < m1; ++m) {
-    if (has0) flux1_march_pair<NS, MIX, EXACT, D, 0, R>(rg, i, r, m, cdt0, p0, s0);
-    if (hasr) flux1_march_pair<NS, MIX, EXACT, D, RA, R>(rg, i, r, m, cdtr, p0, sr);
+      for (int n = 0; n < ncorr1<NS>(); ++n) {
+        const R kl = slot[n * 128];
+        slot[n * 128] = K[n];
+        K[n] = kl;
+      }
+      if (m < m0) continue;
+      flux1_state<NS, EXACT, D, 0, R>(rg, i, j, k, K, p0, ql);
+      flux1_riemann<NS, MIX, EXACT, D, R>(rg, o, i, j, k, ql, qr, p0);
+    }
   }
 }
 
@@ -1221,25 +1208,19 @@ template <int NS, bool MIX, bool EXACT, int D, class R>
 __device__ __forceinline__ void flux1_face(const pcg::StageArgs& a, const pcg::Region& rg, int i, int j, int k) {
   constexpr int O1 = (D == 0) ? 1 : 0;
   constexpr int O2 = (D == 2) ? 1 : 2;
-  const int c[3] = {i, j, k};
   const int di = (D == 0), dj = (D == 1), dk = (D == 2);
   const R p0 = R(p0_of<NS, MIX, R>(rg));
-  // (D|O) exists where the face's O index lies in the box
-  if (c[O1] >= rg.lo[O1] && c[O1] <= rg.hi[O1]) {
-    const R cdt = flux1_cdt<NS, R>(a, rg, O1);
+#pragma unroll(flux1_copies<EXACT, R>())
+  for (int h = 0; h < 2; ++h) {
+    const int o = h == 0 ? O1 : O2;
+    const int c = o == 0 ? i : o == 1 ? j : k;
+    if (c < rg.lo[o] || c > rg.hi[o]) continue;  // (D|O) exists where the face's O index lies in the box
+    const R cdt = flux1_cdt<NS, R>(a, rg, o);
     R ql[pcg::nt_comps(NS)], qr[pcg::nt_comps(NS)];
-    flux1_state_fn<NS, EXACT, D, 0, R>(rg, i, j, k, flux1_corr_fn<NS, O1, R>(rg, i - di, j - dj, k - dk, cdt, p0), p0,
+    flux1_state_fn<NS, EXACT, D, 0, R>(rg, i, j, k, flux1_corr_fn<NS, R>(rg, o, i - di, j - dj, k - dk, cdt, p0), p0,
                                     ql);
-    flux1_state_fn<NS, EXACT, D, 1, R>(rg, i, j, k, flux1_corr_fn<NS, O1, R>(rg, i, j, k, cdt, p0), p0, qr);
-    flux1_riemann<NS, MIX, EXACT, D, O1, R>(rg, i, j, k, ql, qr, p0);
-  }
-  if (c[O2] >= rg.lo[O2] && c[O2] <= rg.hi[O2]) {
-    const R cdt = flux1_cdt<NS, R>(a, rg, O2);
-    R ql[pcg::nt_comps(NS)], qr[pcg::nt_comps(NS)];
-    flux1_state_fn<NS, EXACT, D, 0, R>(rg, i, j, k, flux1_corr_fn<NS, O2, R>(rg, i - di, j - dj, k - dk, cdt, p0), p0,
-                                    ql);
-    flux1_state_fn<NS, EXACT, D, 1, R>(rg, i, j, k, flux1_corr_fn<NS, O2, R>(rg, i, j, k, cdt, p0), p0, qr);
-    flux1_riemann<NS, MIX, EXACT, D, O2, R>(rg, i, j, k, ql, qr, p0);
+    flux1_state_fn<NS, EXACT, D, 1, R>(rg, i, j, k, flux1_corr_fn<NS, R>(rg, o, i, j, k, cdt, p0), p0, qr);
+    flux1_riemann<NS, MIX, EXACT, D, R>(rg, o, i, j, k, ql, qr, p0);
   }
 }
 
