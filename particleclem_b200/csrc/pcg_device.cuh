@@ -131,24 +131,50 @@ __device__ __forceinline__ V4<T> v4(const pcg::View& w) {
   return V4<T>{reinterpret_cast<T*>(w.p), (int)w.js, (int)w.ks, (int)w.ns, w.b[0], w.b[1], w.b[2]};
 }
 
-// A view of a blocked workspace array (pcg::View::blocked, pcg::kCellBlock): cell(i, j, k)
-// is the address of component 0 of the cell; component n is kCellBlock * n elements on.
-template <class T>
+// A view of a blocked workspace array of NC components (pcg::View::blocked,
+// pcg::kCellBlock, pcg::block_vec).
+template <class T, int NC>
 struct B4 {
   T* p;
   int js, ks, bs;
   int bx, by, bz;
-  __device__ __forceinline__ T* cell(int i, int j, int k) const {
-    const int L = (i - bx) + (j - by) * js + (k - bz) * ks;
-    return p + ((L >> 5) * bs + (L & (pcg::kCellBlock - 1)));
-  }
-  __device__ __forceinline__ T& operator()(int i, int j, int k, int n = 0) const {
-    return cell(i, j, k)[n * pcg::kCellBlock];
+  __device__ __forceinline__ int linear(int i, int j, int k) const {
+    return (i - bx) + (j - by) * js + (k - bz) * ks;
   }
 };
-template <class T>
-__device__ __forceinline__ B4<T> b4(const pcg::View& w) {
-  return B4<T>{reinterpret_cast<T*>(w.p), (int)w.js, (int)w.ks, (int)w.ns, w.b[0], w.b[1], w.b[2]};
+template <class T, int NC>
+__device__ __forceinline__ B4<T, NC> b4(const pcg::View& w) {
+  return B4<T, NC>{reinterpret_cast<T*>(w.p), (int)w.js, (int)w.ks, (int)w.ns, w.b[0], w.b[1], w.b[2]};
+}
+
+// V consecutive elements at p (aligned to all of them), one load or store.
+template <int V>
+__device__ __forceinline__ void load_vec(const float* p, float* v) {
+  static_assert(V == 4 || V == 2, "");
+  if constexpr (V == 4) {
+    const float4 w = *reinterpret_cast<const float4*>(p);
+    v[0] = w.x, v[1] = w.y, v[2] = w.z, v[3] = w.w;
+  } else {
+    const float2 w = *reinterpret_cast<const float2*>(p);
+    v[0] = w.x, v[1] = w.y;
+  }
+}
+template <int V>
+__device__ __forceinline__ void load_vec(const double* p, double* v) {
+  static_assert(V == 2, "");
+  const double2 w = *reinterpret_cast<const double2*>(p);
+  v[0] = w.x, v[1] = w.y;
+}
+template <int V>
+__device__ __forceinline__ void store_vec(float* p, const float* v) {
+  if constexpr (V == 4)
+    *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+  else
+    *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
+}
+template <int V>
+__device__ __forceinline__ void store_vec(double* p, const double* v) {
+  *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]);
 }
 
 // ------------------------------------------------------------------ EOS

@@ -21,6 +21,8 @@
 // expression order (parity form) or the reduced algebra (FMA / mixed forms).
 #pragma once
 
+#include <type_traits>
+
 #include "pcg_device.cuh"
 #include "pcg_tma.cuh"
 
@@ -135,19 +137,44 @@ template <class T>
 __device__ __forceinline__ int dstride(const V4<T>& v, int d) {
   return d == 0 ? 1 : d == 1 ? v.js : v.ks;
 }
-// One cell of a blocked view: component n at p[n * kCellBlock] (a compile-time offset).
-template <class T>
+// One cell of a blocked view of NC components.
+template <class T, int NC>
 struct BCell {
-  T* p;
-  __device__ __forceinline__ T& operator[](int n) const { return p[n * pcg::kCellBlock]; }
+  using E = typename std::remove_const<T>::type;
+  static constexpr int V = pcg::block_vec(sizeof(T), NC), NV = NC / V * V;
+  T* g;  // group n0 at g[n0 * kCellBlock]
+  T* t;  // component n past the last whole group at t[n * kCellBlock]
+  // the components n0 .. n0+V-1 (n0 a multiple of V), those below NC
+  __device__ __forceinline__ void get(int n0, E* v) const {
+    if (n0 < NV) {
+      if constexpr (V > 1) load_vec<V>(g + n0 * pcg::kCellBlock, v); else v[0] = g[n0 * pcg::kCellBlock];
+    } else {
+#pragma unroll
+      for (int n = n0; n < NC; ++n) v[n - n0] = t[n * pcg::kCellBlock];
+    }
+  }
+  __device__ __forceinline__ void load(E* v) const {
+#pragma unroll
+    for (int n0 = 0; n0 < NC; n0 += V) get(n0, v + n0);
+  }
+  __device__ __forceinline__ void store(const E* v) const {
+#pragma unroll
+    for (int n0 = 0; n0 < NV; n0 += V) {
+      if constexpr (V > 1) store_vec<V>(g + n0 * pcg::kCellBlock, v + n0); else g[n0 * pcg::kCellBlock] = v[n0];
+    }
+#pragma unroll
+    for (int n = NV; n < NC; ++n) t[n * pcg::kCellBlock] = v[n];
+  }
 };
-template <class T>
-__device__ __forceinline__ BCell<T> at(const B4<T>& v, int i, int j, int k) {
-  return BCell<T>{v.cell(i, j, k)};
+template <class T, int NC>
+__device__ __forceinline__ BCell<T, NC> at(const B4<T, NC>& v, int i, int j, int k) {
+  const int L = v.linear(i, j, k), l = L & (pcg::kCellBlock - 1);
+  T* b = v.p + (L >> 5) * v.bs;
+  return BCell<T, NC>{b + l * BCell<T, NC>::V, b + l};
 }
 // the neighbour of (i, j, k) one cell up in direction d
-template <class T>
-__device__ __forceinline__ BCell<T> at_up(const B4<T>& v, int i, int j, int k, int d) {
+template <class T, int NC>
+__device__ __forceinline__ BCell<T, NC> at_up(const B4<T, NC>& v, int i, int j, int k, int d) {
   return at(v, i + (d == 0), j + (d == 1), k + (d == 2));
 }
 
@@ -481,10 +508,10 @@ __device__ __forceinline__ void trace_ppm_dir(const pcg::Region& rg, const PT& P
     yp2[n] = Ip[2];
   }
 #undef PROFILE3
-  const BCell<R> qp = at(b4<R>(rg.trp[D]), i, j, k);
-  const BCell<R> qm = at(b4<R>(rg.trm[D]), i + (D == 0), j + (D == 1), k + (D == 2));
+  constexpr int NT = pcg::nt_comps(NS);
   // plus state on face i (Source/PPM.cpp:232-331)
   {
+    R q[NT];
     R rho_ref = Imr[0];
     const R un_ref = Imu[0];
     R p_ref = Imp[0];
@@ -509,16 +536,18 @@ __device__ __forceinline__ void trace_ppm_dir(const pcg::Region& rg, const PT& P
     const R rhos = dmax(Lim<R>::tiny(), rho_ref + alphap + alpham + alpha0r);
     const R uns = un_ref + (alphap - alpham) * cc_ref * rho_ref_inv;
     const R ps = dmax(pfloor(Lim<R>::tiny(), p0), p_ref + (alphap + alpham) * csq_ref);
-    qp[pcg::TR_RHO] = rhos;
+    q[pcg::TR_RHO] = rhos;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) qp[pcg::TR_U + c] = (c == D) ? uns : Imt[c];
-    qp[pcg::TR_P] = ps;
+    for (int c = 0; c < 3; ++c) q[pcg::TR_U + c] = (c == D) ? uns : Imt[c];
+    q[pcg::TR_P] = ps;
 #pragma unroll
-    for (int n = 0; n < NS; ++n) qp[pcg::TR_Y + n] = ym1[n];
-    qp[pcg::TR_RE] = EXACT ? rhos * E::ryp2e(rhos, ym1, ps) : ER::rhoe_y(rhos, pabs(ps, p0), ym1);
+    for (int n = 0; n < NS; ++n) q[pcg::TR_Y + n] = ym1[n];
+    q[pcg::TR_RE] = EXACT ? rhos * E::ryp2e(rhos, ym1, ps) : ER::rhoe_y(rhos, pabs(ps, p0), ym1);
+    at(b4<R, NT>(rg.trp[D]), i, j, k).store(q);
   }
   // minus state on face i+1 (Source/PPM.cpp:334-422)
   {
+    R q[NT];
     R rho_ref = Ipr[2];
     const R un_ref = Ipu[2];
     R p_ref = Ipp[2];
@@ -543,17 +572,18 @@ __device__ __forceinline__ void trace_ppm_dir(const pcg::Region& rg, const PT& P
     const R rhos = dmax(Lim<R>::tiny(), rho_ref + alphap + alpham + alpha0r);
     const R uns = un_ref + (alphap - alpham) * cc_ref * rho_ref_inv;
     const R ps = dmax(pfloor(Lim<R>::tiny(), p0), p_ref + (alphap + alpham) * csq_ref);
-    qm[pcg::TR_RHO] = rhos;
+    q[pcg::TR_RHO] = rhos;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) qm[pcg::TR_U + c] = (c == D) ? uns : Ipt[c];
-    qm[pcg::TR_P] = ps;
+    for (int c = 0; c < 3; ++c) q[pcg::TR_U + c] = (c == D) ? uns : Ipt[c];
+    q[pcg::TR_P] = ps;
 #pragma unroll
-    for (int n = 0; n < NS; ++n) qm[pcg::TR_Y + n] = yp1[n];
-    qm[pcg::TR_RE] = EXACT ? rhos * E::ryp2e(rhos, yp1, ps) : ER::rhoe_y(rhos, pabs(ps, p0), yp1);
+    for (int n = 0; n < NS; ++n) q[pcg::TR_Y + n] = yp1[n];
+    q[pcg::TR_RE] = EXACT ? rhos * E::ryp2e(rhos, yp1, ps) : ER::rhoe_y(rhos, pabs(ps, p0), yp1);
+    at_up(b4<R, NT>(rg.trm[D]), i, j, k, D).store(q);
   }
 }
 
-// A traced state held in registers (the low-order boundary faces).
+// A traced state held in registers.
 template <class R>
 struct RegState {
   R* a;
@@ -662,9 +692,13 @@ __device__ __forceinline__ void trace_cell_p(const pcg::StageArgs& a, const pcg:
   const double dt = dt_of(a, rg);
   if (a.ppm_type == 1)
     trace_ppm_dir<NS, MIX, EXACT, HYB, D, R>(rg, P, i, j, k, cc, flat, dt, a.weno_scheme);
-  else
-    plm_cell_p<NS, MIX, D, R>(rg, P, cc, flat, a.plm_iorder, dt, at(b4<R>(rg.trp[D]), i, j, k),
-                              at(b4<R>(rg.trm[D]), i + (D == 0), j + (D == 1), k + (D == 2)));
+  else {
+    constexpr int NT = pcg::nt_comps(NS);
+    R qp[NT], qm[NT];
+    plm_cell_p<NS, MIX, D, R>(rg, P, cc, flat, a.plm_iorder, dt, RegState<R>{qp}, RegState<R>{qm});
+    at(b4<R, NT>(rg.trp[D]), i, j, k).store(qp);
+    at_up(b4<R, NT>(rg.trm[D]), i, j, k, D).store(qm);
+  }
 }
 
 template <int NS, bool MIX, bool EXACT, bool HYB, int D, class R>
@@ -889,12 +923,6 @@ __global__ void __launch_bounds__(128) k_trace_weno(const __grid_constant__ pcg:
 }
 
 // ------------------------------------------------------------------ flux stages
-template <int NS, class R, class C>
-__device__ __forceinline__ void load_state(const C& t, R* s) {
-#pragma unroll
-  for (int n = 0; n < pcg::nt_comps(NS); ++n) s[n] = t[n];
-}
-
 // p0: the region's pressure offset of the FP32 arithmetic (p0_of), formed once by the
 // caller rather than per face (it reads the FP64 state of the region's first cell).
 template <int NS, bool MIX, bool EXACT, int D, class R, bool QX = false>
@@ -910,24 +938,28 @@ __device__ __forceinline__ void face_flux(const pcg::Region& rg, int i, int j, i
                                    gpres, qx);
 }
 
-template <int NS, class R, class C>
-__device__ __forceinline__ void store_tflux(const C& f, const R* fl, R gun, R gpres) {
+template <int NS, class R>
+__device__ __forceinline__ void store_tflux(const pcg::View& w, int i, int j, int k, const R* fl, R gun, R gpres) {
+  constexpr int NF = pcg::nf_comps(NS);
+  R f[NF];
 #pragma unroll
   for (int n = 0; n < 5; ++n) f[n] = fl[n];
 #pragma unroll
   for (int n = 0; n < NS; ++n) f[pcg::FL_Y + n] = fl[pcg::UFS + n];
   f[pcg::FL_Y + NS] = gpres;
   f[pcg::FL_Y + NS + 1] = gun;
+  at(b4<R, NF>(w), i, j, k).store(f);
 }
 
 // First Riemann solves (Source/Godunov.cpp:206-244).
 template <int NS, bool MIX, bool EXACT, int D, class R>
 __device__ __forceinline__ void flux0_face(const pcg::Region& rg, int i, int j, int k) {
-  R ql[pcg::nt_comps(NS)], qr[pcg::nt_comps(NS)], fl[pcg::nvar(NS)], gun, gpres;
-  load_state<NS, R>(at(b4<R>(rg.trm[D]), i, j, k), ql);
-  load_state<NS, R>(at(b4<R>(rg.trp[D]), i, j, k), qr);
+  constexpr int NT = pcg::nt_comps(NS);
+  R ql[NT], qr[NT], fl[pcg::nvar(NS)], gun, gpres;
+  at(b4<const R, NT>(rg.trm[D]), i, j, k).load(ql);
+  at(b4<const R, NT>(rg.trp[D]), i, j, k).load(qr);
   face_flux<NS, MIX, EXACT, D, R>(rg, i, j, k, ql, qr, R(p0_of<NS, MIX, R>(rg)), fl, gun, gpres);
-  store_tflux<NS, R>(at(b4<R>(rg.fi[D]), i, j, k), fl, gun, gpres);
+  store_tflux<NS, R>(rg.fi[D], i, j, k, fl, gun, gpres);
 }
 
 template <int NS, bool MIX, bool EXACT, class R, int MINB>
@@ -965,74 +997,60 @@ __device__ __forceinline__ bool march_of(const pcg::Seg& sg, int t, int& i, int&
 // and transdo_apply corrects one traced state with it, by the reference's expressions.
 template <int NS> constexpr int ncorr1() { return 6 + NS; }
 
-// The O-correction of one cell formed on demand from its two O-fluxes (component n of K).
-template <int NS, class R, class C = BCell<const R>>
-struct TransdoCorr {
-  C f, g;  // the cell's first O-fluxes on its low and high O-faces
-  R cdtdx, c, p0;
-  __device__ __forceinline__ R operator()(int n) const {
-    if (n < pcg::FL_Y + NS) return cdtdx * (g[n] - f[n]);
-    const R pggp = g[pcg::FL_Y + NS];
-    const R pggm = f[pcg::FL_Y + NS];
-    const R ugp = g[pcg::FL_Y + NS + 1];
-    const R ugm = f[pcg::FL_Y + NS + 1];
-    const R dAup = pggp * ugp - pggm * ugm;
-    const R pav = R(0.5) * (pggp + pggm);
-    const R dAu = ugp - ugm;
-    R dpt = dAup + pav * dAu * (c - R(1));
-    if constexpr (PDev<R>::on) dpt = dpt + p0 * c * dAu;
-    return cdtdx * dpt;
-  }
-};
-// A correction already formed (K[n]).
-template <class R>
-struct CorrArray {
-  const R* K;
-  __device__ __forceinline__ R operator()(int n) const { return K[n]; }
-};
-
+// f and g are the cell's first O-fluxes on its low and high O-faces.
 template <int NS, class R, class C>
-__device__ __forceinline__ void transdo_corr(const C& f, const C& g, R cdtdx, R c, R p0, R* K) {
-  const TransdoCorr<NS, R, C> kc{f, g, cdtdx, c, p0};
-  constexpr int NC = pcg::FL_Y + NS;
-  if constexpr (sizeof(R) == 4) {
-    // the flux differences in component pairs with packed FP32 (FMUL2)
-    const float2 c2 = make_float2(cdtdx, cdtdx);
+__device__ __forceinline__ void transdo_corr(const C& fc, const C& gc, R cdtdx, R c, R p0, R* K) {
+  constexpr int NC = pcg::FL_Y + NS, NF = pcg::nf_comps(NS);
+  R f[NF], g[NF];
 #pragma unroll
-    for (int m = 0; m < NC / 2; ++m) {
-      const int n = 2 * m;
-      const float2 v = __fmul2_rn(c2, __fadd2_rn(make_float2(g[n], g[n + 1]), make_float2(-f[n], -f[n + 1])));
-      K[n] = v.x;
-      K[n + 1] = v.y;
+  for (int n0 = 0; n0 < NF; n0 += C::V) {
+    fc.get(n0, f + n0);
+    gc.get(n0, g + n0);
+    if constexpr (sizeof(R) == 4) {
+      // the flux differences in component pairs with packed FP32 (FMUL2)
+      const float2 c2 = make_float2(cdtdx, cdtdx);
+#pragma unroll
+      for (int n = n0; n < n0 + C::V; n += 2) {
+        if (n + 1 < NC) {
+          const float2 v = __fmul2_rn(c2, __fadd2_rn(make_float2(g[n], g[n + 1]), make_float2(-f[n], -f[n + 1])));
+          K[n] = v.x;
+          K[n + 1] = v.y;
+        } else if (n < NC) {
+          K[n] = cdtdx * (g[n] - f[n]);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int n = n0; n < n0 + C::V; ++n)
+        if (n < NC) K[n] = cdtdx * (g[n] - f[n]);
     }
-    if constexpr (NC % 2) K[NC - 1] = kc(NC - 1);
-    K[NC] = kc(NC);
-  } else {
-#pragma unroll
-    for (int n = 0; n < ncorr1<NS>(); ++n) K[n] = kc(n);
   }
+  const R pggp = g[NC], pggm = f[NC], ugp = g[NC + 1], ugm = f[NC + 1];
+  const R dAup = pggp * ugp - pggm * ugm;
+  const R pav = R(0.5) * (pggp + pggm);
+  const R dAu = ugp - ugm;
+  R dpt = dAup + pav * dAu * (c - R(1));
+  if constexpr (PDev<R>::on) dpt = dpt + p0 * c * dAu;
+  K[NC] = cdtdx * dpt;
 }
 
-template <int NS, bool EXACT, class R, class KF>
-__device__ __forceinline__ void transdo_apply(const R* qn, const KF& K, R p0, R* out) {
-  const R flxrho = K(0);
-  const R flxu = K(1);
-  const R flxv = K(2);
-  const R flxw = K(3);
-  const R flxe = K(4);
+template <int NS, bool EXACT, class R>
+__device__ __forceinline__ void transdo_apply(const R* qn, const R* K, R p0, R* out) {
+  const R flxrho = K[0];
+  const R flxu = K[1];
+  const R flxv = K[2];
+  const R flxw = K[3];
+  const R flxe = K[4];
   const R rr = qn[pcg::TR_RHO];
   const R rrnew = rr - flxrho;
   const R irrnew = EXACT ? R(0) : rrcp(rrnew);
   R num[NS + 4];  // EXACT: the numerators over rrnew, divided together
   if constexpr (sizeof(R) == 4 && NS > 1) {
-    R kc[NS];
-#pragma unroll
-    for (int n = 0; n < NS; n++) kc[n] = K(pcg::FL_Y + n);
-    scale_sub2<NS>(rr, qn + pcg::TR_Y, kc, irrnew, out + pcg::TR_Y);
+    scale_sub2<NS>(rr, qn + pcg::TR_Y, K + pcg::FL_Y, irrnew, out + pcg::TR_Y);
   } else {
 #pragma unroll
     for (int n = 0; n < NS; n++) {
-      const R compn = K(pcg::FL_Y + n);
+      const R compn = K[pcg::FL_Y + n];
       num[n] = rr * qn[pcg::TR_Y + n] - compn;
       if (!EXACT) out[pcg::TR_Y + n] = num[n] * irrnew;
     }
@@ -1063,7 +1081,7 @@ __device__ __forceinline__ void transdo_apply(const R* qn, const KF& K, R p0, R*
   out[pcg::TR_W] = EXACT ? num[NS + 2] : rwnew * irrnew;
   const R rhoekin = EXACT ? num[NS + 3] : R(0.5) * ke2 * irrnew;
   out[pcg::TR_RE] = renew - rhoekin;
-  const R pnew = qn[pcg::TR_P] - K(5 + NS);
+  const R pnew = qn[pcg::TR_P] - K[5 + NS];
   out[pcg::TR_P] = dmax(pnew, pfloor(Lim<R>::very_small(), p0));
 }
 
@@ -1079,31 +1097,19 @@ template <bool EXACT, class R> constexpr int flux1_copies() { return !EXACT && s
 // its gamma_c.
 template <int NS, class R>
 __device__ __forceinline__ void flux1_corr(const pcg::Region& rg, int o, int i, int j, int k, R cdt, R p0, R* K) {
-  const B4<const R> fov = b4<const R>(rg.fi[o]);
+  const auto fov = b4<const R, pcg::nf_comps(NS)>(rg.fi[o]);
   const R c = R(v4<const double>(rg.qa)(i, j, k, pcg::QGAMC));
   transdo_corr<NS, R>(at(fov, i, j, k), at_up(fov, i, j, k, o), cdt, c, p0, K);
 }
 
 // The (D|O) flux at the D-face (i, j, k) from the left and right O-corrections
 // (Source/Godunov.cpp:246-384).
-template <int NS, bool EXACT, int D, int SIDE, class R, class KF>
-__device__ __forceinline__ void flux1_state_fn(const pcg::Region& rg, int i, int j, int k, const KF& K, R p0, R* q) {
-  R qn[pcg::nt_comps(NS)];
-  load_state<NS, R>(at(b4<R>(SIDE == 0 ? rg.trm[D] : rg.trp[D]), i, j, k), qn);
-  transdo_apply<NS, EXACT, R>(qn, K, p0, q);
-}
 template <int NS, bool EXACT, int D, int SIDE, class R>
 __device__ __forceinline__ void flux1_state(const pcg::Region& rg, int i, int j, int k, const R* K, R p0, R* q) {
-  flux1_state_fn<NS, EXACT, D, SIDE, R>(rg, i, j, k, CorrArray<R>{K}, p0, q);
-}
-
-// The O-correction of the cell (i, j, k), formed on demand.
-template <int NS, class R>
-__device__ __forceinline__ TransdoCorr<NS, R> flux1_corr_fn(const pcg::Region& rg, int o, int i, int j, int k, R cdt,
-                                                            R p0) {
-  const B4<const R> fov = b4<const R>(rg.fi[o]);
-  return TransdoCorr<NS, R>{at(fov, i, j, k), at_up(fov, i, j, k, o), cdt,
-                            R(v4<const double>(rg.qa)(i, j, k, pcg::QGAMC)), p0};
+  constexpr int NT = pcg::nt_comps(NS);
+  R qn[NT];
+  at(b4<const R, NT>(SIDE == 0 ? rg.trm[D] : rg.trp[D]), i, j, k).load(qn);
+  transdo_apply<NS, EXACT, R>(qn, K, p0, q);
 }
 
 template <int NS, bool MIX, bool EXACT, int D, class R>
@@ -1111,7 +1117,7 @@ __device__ __forceinline__ void flux1_riemann(const pcg::Region& rg, int o, int 
                                               const R* qr, R p0) {
   R fl[pcg::nvar(NS)], gun, gpres;
   face_flux<NS, MIX, EXACT, D, R>(rg, i, j, k, ql, qr, p0, fl, gun, gpres);
-  store_tflux<NS, R>(at(b4<R>(rg.fdo[D][o]), i, j, k), fl, gun, gpres);
+  store_tflux<NS, R>(rg.fdo[D][o], i, j, k, fl, gun, gpres);
 }
 
 template <int NS, class R>
@@ -1202,8 +1208,7 @@ __device__ __forceinline__ void flux1_march(const pcg::StageArgs& a, const pcg::
 }
 
 // FP64 forms: one D-face per thread, both corrections of each pair formed by the
-// thread component by component as the state update consumes them (in FP64 the
-// shared forms above hold more registers than they save).
+// thread (in FP64 the shared forms above hold more registers than they save).
 template <int NS, bool MIX, bool EXACT, int D, class R>
 __device__ __forceinline__ void flux1_face(const pcg::StageArgs& a, const pcg::Region& rg, int i, int j, int k) {
   constexpr int O1 = (D == 0) ? 1 : 0;
@@ -1216,10 +1221,11 @@ __device__ __forceinline__ void flux1_face(const pcg::StageArgs& a, const pcg::R
     const int c = o == 0 ? i : o == 1 ? j : k;
     if (c < rg.lo[o] || c > rg.hi[o]) continue;  // (D|O) exists where the face's O index lies in the box
     const R cdt = flux1_cdt<NS, R>(a, rg, o);
-    R ql[pcg::nt_comps(NS)], qr[pcg::nt_comps(NS)];
-    flux1_state_fn<NS, EXACT, D, 0, R>(rg, i, j, k, flux1_corr_fn<NS, R>(rg, o, i - di, j - dj, k - dk, cdt, p0), p0,
-                                    ql);
-    flux1_state_fn<NS, EXACT, D, 1, R>(rg, i, j, k, flux1_corr_fn<NS, R>(rg, o, i, j, k, cdt, p0), p0, qr);
+    R K[ncorr1<NS>()], ql[pcg::nt_comps(NS)], qr[pcg::nt_comps(NS)];
+    flux1_corr<NS, R>(rg, o, i - di, j - dj, k - dk, cdt, p0, K);
+    flux1_state<NS, EXACT, D, 0, R>(rg, i, j, k, K, p0, ql);
+    flux1_corr<NS, R>(rg, o, i, j, k, cdt, p0, K);
+    flux1_state<NS, EXACT, D, 1, R>(rg, i, j, k, K, p0, qr);
     flux1_riemann<NS, MIX, EXACT, D, R>(rg, o, i, j, k, ql, qr, p0);
   }
 }
@@ -1261,25 +1267,36 @@ __global__ void __launch_bounds__(128, MINB) k_flux1(const __grid_constant__ pcg
 template <int NS> constexpr int ncorr() { return 7 + NS; }
 
 template <int NS, class R, class C>
-__device__ __forceinline__ void transdd_corr(const C& fx, const C& gx, const C& fy, const C& gy, R cdtdx0, R cdtdx1,
-                                             R c, R p0, R* K) {
-  constexpr int NC = pcg::FL_Y + NS;
-  if constexpr (sizeof(R) == 4) {
-    // component pairs with packed FP32 (FFMA2)
-    const float2 c0 = make_float2(cdtdx0, cdtdx0), c1 = make_float2(cdtdx1, cdtdx1);
+__device__ __forceinline__ void transdd_corr(const C& fxc, const C& gxc, const C& fyc, const C& gyc, R cdtdx0,
+                                             R cdtdx1, R c, R p0, R* K) {
+  constexpr int NC = pcg::FL_Y + NS, NF = pcg::nf_comps(NS);
+  R fx[NF], gx[NF], fy[NF], gy[NF];
 #pragma unroll
-    for (int m = 0; m < NC / 2; ++m) {
-      const int n = 2 * m;
-      const float2 dx = __fadd2_rn(make_float2(gx[n], gx[n + 1]), make_float2(-fx[n], -fx[n + 1]));
-      const float2 dy = __fadd2_rn(make_float2(gy[n], gy[n + 1]), make_float2(-fy[n], -fy[n + 1]));
-      const float2 v = __ffma2_rn(c0, dx, __fmul2_rn(c1, dy));
-      K[n] = v.x;
-      K[n + 1] = v.y;
+  for (int n0 = 0; n0 < NF; n0 += C::V) {
+    fxc.get(n0, fx + n0);
+    gxc.get(n0, gx + n0);
+    fyc.get(n0, fy + n0);
+    gyc.get(n0, gy + n0);
+    if constexpr (sizeof(R) == 4) {
+      // component pairs with packed FP32 (FFMA2)
+      const float2 c0 = make_float2(cdtdx0, cdtdx0), c1 = make_float2(cdtdx1, cdtdx1);
+#pragma unroll
+      for (int n = n0; n < n0 + C::V; n += 2) {
+        if (n + 1 < NC) {
+          const float2 dx = __fadd2_rn(make_float2(gx[n], gx[n + 1]), make_float2(-fx[n], -fx[n + 1]));
+          const float2 dy = __fadd2_rn(make_float2(gy[n], gy[n + 1]), make_float2(-fy[n], -fy[n + 1]));
+          const float2 v = __ffma2_rn(c0, dx, __fmul2_rn(c1, dy));
+          K[n] = v.x;
+          K[n + 1] = v.y;
+        } else if (n < NC) {
+          K[n] = cdtdx0 * (gx[n] - fx[n]) + cdtdx1 * (gy[n] - fy[n]);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int n = n0; n < n0 + C::V; ++n)
+        if (n < NC) K[n] = cdtdx0 * (gx[n] - fx[n]) + cdtdx1 * (gy[n] - fy[n]);
     }
-    if constexpr (NC % 2) K[NC - 1] = cdtdx0 * (gx[NC - 1] - fx[NC - 1]) + cdtdx1 * (gy[NC - 1] - fy[NC - 1]);
-  } else {
-#pragma unroll
-    for (int n = 0; n < NC; ++n) K[n] = cdtdx0 * (gx[n] - fx[n]) + cdtdx1 * (gy[n] - fy[n]);
   }
   const int gp = pcg::FL_Y + NS, gu = pcg::FL_Y + NS + 1;
   const R dAupx = gx[gp] * gx[gu] - fx[gp] * fx[gu];
@@ -1388,8 +1405,8 @@ __device__ __forceinline__ void flux2_corr(const pcg::Region& rg, int i, int j, 
                                            R* K) {
   constexpr int O1 = (D == 0) ? 1 : 0;
   constexpr int O2 = (D == 2) ? 1 : 2;
-  const B4<const R> fxv = b4<const R>(rg.fdo[O1][O2]);
-  const B4<const R> fyv = b4<const R>(rg.fdo[O2][O1]);
+  const auto fxv = b4<const R, pcg::nf_comps(NS)>(rg.fdo[O1][O2]);
+  const auto fyv = b4<const R, pcg::nf_comps(NS)>(rg.fdo[O2][O1]);
   const R c = R(v4<const double>(rg.qa)(i, j, k, pcg::QGAMC));
   transdd_corr<NS, R>(at(fxv, i, j, k), at_up(fxv, i, j, k, O1), at(fyv, i, j, k), at_up(fyv, i, j, k, O2), cdtdx0,
                       cdtdx1, c, p0, K);
@@ -1404,8 +1421,9 @@ __device__ __forceinline__ void flux2_state(const pcg::Region& rg, int i, int j,
   const V4<const double> sqv = v4<const double>(rg.srcq);
   CellPtr<const double> sq = has_src ? at(sqv, i, j, k) : CellPtr<const double>{nullptr, 0};
   if (SIDE == 0 && has_src) sq = shift(sq, -dstride(sqv, D));
-  R qn[pcg::nt_comps(NS)];
-  load_state<NS, R>(at(b4<R>(SIDE == 0 ? rg.trm[D] : rg.trp[D]), i, j, k), qn);
+  constexpr int NT = pcg::nt_comps(NS);
+  R qn[NT];
+  at(b4<const R, NT>(SIDE == 0 ? rg.trm[D] : rg.trp[D]), i, j, k).load(qn);
   transdd_apply<NS, EXACT, R>(qn, K, hdt, has_src, sq, p0, q);
 }
 
@@ -1473,12 +1491,12 @@ __device__ __forceinline__ void flux2_face(const pcg::StageArgs& a, const pcg::R
       flr[pcg::UTEMP] = 0.f;
       adjust_fluxes<NS, D, float>(flr, u, ud, visc, at_bndry);
       const float arf = float(ar);
-      const BCell<float> ff = at(b4<float>(rg.ff[D]), i, j, k);
+      constexpr int NV = pcg::nvar(NS);
 #pragma unroll
-      for (int n = 0; n < pcg::nvar(NS); ++n) ff[n] = flr[n] * arf;
-      const BCell<float> qe = at(b4<float>(rg.qec[D]), i, j, k);
-      qe[0] = float(gpres);
-      qe[1] = float(gun);
+      for (int n = 0; n < NV; ++n) flr[n] *= arf;
+      at(b4<float, NV>(rg.ff[D]), i, j, k).store(flr);
+      const float qe[2] = {float(gpres), float(gun)};
+      at(b4<float, 2>(rg.qec[D]), i, j, k).store(qe);
       return;
     }
   }
@@ -1727,21 +1745,37 @@ __global__ void __launch_bounds__(128) k_srctoprim(const __grid_constant__ pcg::
 // the Godunov pressures of pdivu).
 // The final fluxes and face states of the cell's six faces: FP64 arrays (caller's or
 // workspace, Array4 layout) or the mixed form's FP32 workspace arrays (blocked layout).
-template <class F> struct FinalView;
-template <> struct FinalView<double> {
-  using C = CellPtr<const double>;
-  static __device__ __forceinline__ void cells(const pcg::View& w, int d, int i, int j, int k, C& lo, C& hi) {
+// One face's NC values, read V at a time.
+template <class F, int NC> struct FinalView;
+template <int NC> struct FinalView<double, NC> {
+  static constexpr int V = 1;
+  CellPtr<const double> lo, hi;
+  __device__ __forceinline__ FinalView(const pcg::View& w, int d, int i, int j, int k) {
     const V4<const double> v = v4<const double>(w);
     lo = at(v, i, j, k);
     hi = shift(lo, dstride(v, d));
   }
+  __device__ __forceinline__ void get(int n0, double* a, double* b) const {
+    a[0] = lo[n0];
+    b[0] = hi[n0];
+  }
 };
-template <> struct FinalView<float> {
-  using C = BCell<const float>;
-  static __device__ __forceinline__ void cells(const pcg::View& w, int d, int i, int j, int k, C& lo, C& hi) {
-    const B4<const float> v = b4<const float>(w);
+template <int NC> struct FinalView<float, NC> {
+  using C = BCell<const float, NC>;
+  static constexpr int V = C::V;
+  C lo, hi;
+  __device__ __forceinline__ FinalView(const pcg::View& w, int d, int i, int j, int k) {
+    const auto v = b4<const float, NC>(w);
     lo = at(v, i, j, k);
     hi = at_up(v, i, j, k, d);
+  }
+  __device__ __forceinline__ void get(int n0, double* a, double* b) const {
+    float x[V], y[V];
+    lo.get(n0, x);
+    hi.get(n0, y);
+#pragma unroll
+    for (int m = 0; m < V; ++m)
+      if (n0 + m < NC) a[m] = double(x[m]), b[m] = double(y[m]);
   }
 };
 
@@ -1750,14 +1784,17 @@ template <> struct FinalView<float> {
 // component as it is formed instead of holding all of them.
 template <int NS, class F, class OUT>
 __device__ __forceinline__ void consup_each(const pcg::Region& rg, int i, int j, int k, double p0, OUT&& out) {
-  using FV = FinalView<F>;
-  typename FV::C f0, f0p, f1, f1p, f2, f2p, q0, q0p, q1, q1p, q2, q2p;
-  FV::cells(rg.ff[0], 0, i, j, k, f0, f0p);
-  FV::cells(rg.ff[1], 1, i, j, k, f1, f1p);
-  FV::cells(rg.ff[2], 2, i, j, k, f2, f2p);
-  FV::cells(rg.qec[0], 0, i, j, k, q0, q0p);
-  FV::cells(rg.qec[1], 1, i, j, k, q1, q1p);
-  FV::cells(rg.qec[2], 2, i, j, k, q2, q2p);
+  constexpr int NV = pcg::nvar(NS);
+  const FinalView<F, NV> f0(rg.ff[0], 0, i, j, k), f1(rg.ff[1], 1, i, j, k), f2(rg.ff[2], 2, i, j, k);
+  const FinalView<F, 2> e0(rg.qec[0], 0, i, j, k), e1(rg.qec[1], 1, i, j, k), e2(rg.qec[2], 2, i, j, k);
+  constexpr int VE = FinalView<F, 2>::V;
+  double q0[2], q0p[2], q1[2], q1p[2], q2[2], q2p[2];
+#pragma unroll
+  for (int n0 = 0; n0 < 2; n0 += VE) {
+    e0.get(n0, q0 + n0, q0p + n0);
+    e1.get(n0, q1 + n0, q1p + n0);
+    e2.get(n0, q2 + n0, q2p + n0);
+  }
   const bool ua = rg.area[0].p != nullptr;
   const V4<const double> a0 = v4<const double>(rg.area[0]);
   const V4<const double> a1 = v4<const double>(rg.area[1]);
@@ -1767,14 +1804,21 @@ __device__ __forceinline__ void consup_each(const pcg::Region& rg, int i, int j,
   const double a2m = ua ? a2(i, j, k) : rg.area_u[2], a2p = ua ? a2(i, j, k + 1) : rg.area_u[2];
   const double v = rg.vol.p ? v4<const double>(rg.vol)(i, j, k) : rg.vol_u;
   // the volume divides every component's flux sum and the p div u term: divided together
-  constexpr int NV = pcg::nvar(NS);
+  constexpr int V = FinalView<F, NV>::V;
   double num[NV + 1];
 #pragma unroll
-  for (int n = 0; n < NV; ++n)
-    num[n] = double(f0[n]) - double(f0p[n]) + double(f1[n]) - double(f1p[n]) + double(f2[n]) - double(f2p[n]);
-  num[NV] = 0.5 * ((double(q0p[0]) + p0 + (double(q0[0]) + p0)) * (double(q0p[1]) * a0p - double(q0[1]) * a0m) +
-                   (double(q1p[0]) + p0 + (double(q1[0]) + p0)) * (double(q1p[1]) * a1p - double(q1[1]) * a1m) +
-                   (double(q2p[0]) + p0 + (double(q2[0]) + p0)) * (double(q2p[1]) * a2p - double(q2[1]) * a2m));
+  for (int n0 = 0; n0 < NV; n0 += V) {
+    double xm[V], xp[V], ym[V], yp[V], zm[V], zp[V];
+    f0.get(n0, xm, xp);
+    f1.get(n0, ym, yp);
+    f2.get(n0, zm, zp);
+#pragma unroll
+    for (int m = 0; m < V; ++m)
+      if (n0 + m < NV) num[n0 + m] = xm[m] - xp[m] + ym[m] - yp[m] + zm[m] - zp[m];
+  }
+  num[NV] = 0.5 * ((q0p[0] + p0 + (q0[0] + p0)) * (q0p[1] * a0p - q0[1] * a0m) +
+                   (q1p[0] + p0 + (q1[0] + p0)) * (q1p[1] * a1p - q1[1] * a1m) +
+                   (q2p[0] + p0 + (q2[0] + p0)) * (q2p[1] * a2p - q2[1] * a2m));
   div_all<NV + 1>(num, v, num);
   const CellPtr<double> uo = at(v4<double>(rg.uout), i, j, k);
 #pragma unroll

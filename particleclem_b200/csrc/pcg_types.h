@@ -82,11 +82,17 @@ struct EosConst {
 // kernel that reads it): p[(i-b0) + (j-b1)*js + (k-b2)*ks + n*ns].
 // Blocked workspace arrays (the traced states and the face fluxes the flux stages pass
 // on) use the same linear cell index L = (i-b0) + (j-b1)*js + (k-b2)*ks but group the
-// cells in blocks of kCellBlock consecutive L, each block holding all its components one
-// after the other: element (L, n) at p[(L / 32) * ns + n * 32 + L % 32], ns = 32 * ncomp.
-// A warp reading one component of 32 consecutive cells still reads 128 contiguous bytes,
-// and the components of a cell are compile-time offsets from its first one.
+// cells in blocks of kCellBlock consecutive L, each block holding all its components
+// (ns = 32 * ncomp elements) in groups of block_vec = V: the V components n0 .. n0+V-1 of a
+// cell are V consecutive elements at p[(L / 32) * ns + n0 * 32 + V * (L % 32)], 16 bytes, which
+// one load or store moves; the ncomp % V components after the last whole group follow one
+// after the other, component n at p[(L / 32) * ns + n * 32 + L % 32]. A warp still moves whole
+// lines, and every component of a cell is at a compile-time offset from two addresses.
 constexpr int kCellBlock = 32;
+PCG_HD constexpr int block_vec(size_t esz, int ncomp) {
+  const int v = int(16 / esz);
+  return ncomp >= v ? v : ncomp >= 2 ? 2 : 1;
+}
 struct View {
   void* p;
   int64_t js, ks, ns;
