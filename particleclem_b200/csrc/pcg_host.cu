@@ -536,6 +536,25 @@ void reverse_segs(Layout& L, int stage) {
   }
 }
 
+// Order the segments of a stage by direction (x of every region, then y, then z), block
+// offsets renumbered. Each direction is its own code, and with a few blocks of every region
+// resident all three compete for an SM's instruction caches. 64 boxes of 32^3, 9 species, FP64:
+// flux0 0.795 -> 0.717 ms, flux1 2.25 -> 2.07, flux2 1.72 -> 1.48; the trace, whose directions
+// share the primitives they read, 1.478 -> 1.504, so it keeps its order.
+void group_segs(Layout& L, int stage) {
+  std::vector<pcg::Seg>& v = L.segs[stage];
+  const size_t n = v.size();
+  std::vector<std::pair<pcg::Seg, int64_t>> w(n);
+  for (size_t i = 0; i < n; ++i) w[i] = {v[i], (i + 1 < n ? v[i + 1].blk0 : L.nblocks[stage]) - v[i].blk0};
+  std::stable_sort(w.begin(), w.end(), [](const auto& a, const auto& b) { return a.first.variant < b.first.variant; });
+  int64_t b = 0;
+  for (size_t i = 0; i < n; ++i) {
+    v[i] = w[i].first;
+    v[i].blk0 = b;
+    b += w[i].second;
+  }
+}
+
 // The tiled trace of direction d over g1 = grow(box,1), as K_TRACE_TILE segments: the up
 // to three disjoint strips that full tiles cannot cover, along x, y and z (variant d:
 // one cell per thread, read from global memory), and the full tiles of the rest
@@ -721,6 +740,8 @@ void build_layout(Layout& L, const std::vector<BoxIn>& boxes, const pcg_hydro_pa
     add_seg(L, K_CONSUP, (int)r, 0, B.bx);
     L.regions.push_back(R);
   }
+  if (boxes.size() > 1)
+    for (int st : {K_FLUX0, K_FLUX1, K_FLUX2}) group_segs(L, st);
   // alternate traversal directions of successive stages (see add_dir_segs); K_CONSUP
   // keeps one segment per region in region order (the per-box timesteps index it)
   for (int st = K_CTOPRIM; st <= K_FLUX2; ++st)
