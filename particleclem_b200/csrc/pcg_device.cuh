@@ -676,34 +676,29 @@ __device__ __forceinline__ R flatten(const Q& q, int i, int j, int k, int dir) {
   const R zcut1 = R(0.75e0);
   const R zcut2 = R(0.85e0);
   const R dzcut = R(1) / (zcut2 - zcut1);
+  // chi z of the cell at offset o (0: this cell, -ishft: the upstream one): zero unless the
+  // flow converges there and the pressure jumps by a third of its lower value. The jump test
+  // is settled without its division where |dp| <= 0.3 of a positive lower value (far below
+  // the threshold 0.33), and the steepness z, which lies in [0, 1] even for NaN, is formed
+  // (its two outer pressures read) only where the test holds.
+  const auto chi_z = [&](int o, R qp, R qm, R dp) {
+    if (!(QS(o - 1, pcg::QU + dir) - QS(o + 1, pcg::QU + dir) >= R(0))) return R(0);
+    const R tmp = dmin(qp, qm);
+    if (tmp > R(0) && fabs(dp) <= R(0.3) * tmp) return R(0);
+    if (!((fabs(dp) / tmp) > shktst)) return R(0);
+    const R denom = dmax(small_pres, fabs(QS(o + 2, n) - QS(o - 2, n)));
+    const R zeta = fabs(dp) / denom;
+    return min1_max0<R>(dzcut * (zeta - zcut1));
+  };
   const R qm = QS(-1, n);
   const R qp = QS(1, n);
-  const R qmun = QS(-1, pcg::QU + dir);
-  const R qpun = QS(1, pcg::QU + dir);
-  const R qmm = QS(-2, n);
-  const R qpp = QS(2, n);
-  R dp = qp - qm;
+  const R dp = qp - qm;
   const int ishft = (dp > R(0)) ? 1 : -1;
-  R denom = dmax(small_pres, fabs(qpp - qmm));
-  R zeta = fabs(dp) / denom;
-  const R z = min1_max0<R>(dzcut * (zeta - zcut1));
-  R tst = (qmun - qpun >= R(0)) ? R(1) : R(0);
-  R tmp = dmin(qp, qm);
-  const R chi = (fabs(dp) / tmp) > shktst ? tst : R(0);
+  const R here = chi_z(0, qp, qm, dp);
   const R qpshft = QS(1 - ishft, n);
   const R qmshft = QS(-(1 + ishft), n);
-  const R qpunshft = QS(1 - ishft, pcg::QU + dir);
-  const R qmunshft = QS(-(1 + ishft), pcg::QU + dir);
-  const R qppshft = QS(2 - ishft, n);
-  const R qmmshft = QS(-(2 + ishft), n);
-  dp = qpshft - qmshft;
-  denom = dmax(small_pres, fabs(qppshft - qmmshft));
-  zeta = fabs(dp) / denom;
-  const R z2 = min1_max0<R>(dzcut * (zeta - zcut1));
-  tst = (qmunshft - qpunshft >= R(0)) ? R(1) : R(0);
-  tmp = dmin(qpshft, qmshft);
-  const R chi2 = (fabs(dp) / tmp) > shktst ? tst : R(0);
-  return R(1) - dmax(chi2 * z2, chi * z);
+  const R there = chi_z(-ishft, qpshft, qmshft, qpshft - qmshft);
+  return R(1) - dmax(there, here);
 #undef QS
 }
 
