@@ -605,7 +605,8 @@ __device__ __forceinline__ R vl_slope(R a, R b, R c) {
   R s = R(0);
   if (dsl * dsr > R(0)) {
     const R dsc = R(0.5) * (c - a);
-    s = copysign(R(1), dsc) * dmin(fabs(dsc), dmin(fabs(dsl), fabs(dsr)));
+    // the reference's sign(dsc) * min(...), the sign set instead of multiplied in
+    s = copysign(dmin(fabs(dsc), dmin(fabs(dsl), fabs(dsr))), dsc);
   }
   return s;
 }
@@ -647,15 +648,37 @@ __device__ __forceinline__ void ppm_reconstruct(const R s0, const R s1, const R 
   ppm_limit(s2, flatn, sm, sp);
 }
 
-// Source/PPM.H:131-189 (ppm_int_profile), one wave
+// Source/PPM.H:131-189 (ppm_int_profile), one wave:
+//   speed <= 0:  Im = sm + h (sp - sm + b s6),  Ip = sp
+//   speed > 0:   Ip = sp - h (sp - sm - b s6),  Im = sm
+// with h = sigma / 2, b = 1 - 2 sigma / 3. In FP32 the signs go into the wave's h and b, so that
+// one expression serves both sides of every component (the same roundings: only signs move);
+// 256^3 one-species trace 2.00 -> 1.92 ms. In FP64 the branch measured faster (1.46 against 1.49
+// ms, 9 species at 128^3).
 template <class R>
-__device__ __forceinline__ void ppm_wave(R sm, R sp, R s6, R speed, R dtdx, R& Ip, R& Im) {
+struct PpmWave {
+  bool left;  // speed <= 0
+  R h, b;
+};
+template <class R>
+__device__ __forceinline__ PpmWave<R> ppm_wave_of(R speed, R dtdx) {
   const R sigma = fabs(speed) * dtdx;
-  if (speed <= R(0)) {
+  const R h = R(0.5) * sigma, b = R(1) - (R(2) / R(3)) * sigma;
+  const bool left = speed <= R(0);
+  if constexpr (sizeof(R) == 4) return PpmWave<R>{left, left ? h : -h, left ? b : -b};
+  return PpmWave<R>{left, h, b};
+}
+template <class R>
+__device__ __forceinline__ void ppm_wave(R sm, R sp, R s6, const PpmWave<R>& w, R& Ip, R& Im) {
+  if constexpr (sizeof(R) == 4) {
+    const R v = (w.left ? sm : sp) + w.h * (sp - sm + w.b * s6);
+    Ip = w.left ? sp : v;
+    Im = w.left ? v : sm;
+  } else if (w.left) {
     Ip = sp;
-    Im = sm + R(0.5) * sigma * (sp - sm + (R(1) - (R(2) / R(3)) * sigma) * s6);
+    Im = sm + w.h * (sp - sm + w.b * s6);
   } else {
-    Ip = sp - R(0.5) * sigma * (sp - sm - (R(1) - (R(2) / R(3)) * sigma) * s6);
+    Ip = sp - w.h * (sp - sm - w.b * s6);
     Im = sm;
   }
 }
@@ -706,28 +729,25 @@ __device__ __forceinline__ R flatten(const Q& q, int i, int j, int k, int dir) {
 template <class R>
 __device__ __forceinline__ R plm_slope(R qm2, R qm, R qc, R qp, R qp2, R flat, int order) {
   if (order == 1) return R(0);
-  R dlft, drgt, dcen, dfm = R(0), dfp = R(0), dlim, dsgn, dtemp;
+  R dlft, drgt, dcen, dfm = R(0), dfp = R(0), dlim, dtemp;
   if (order == 4) {
     dlft = qm - qm2;
     drgt = qc - qm;
     dcen = R(0.5) * (dlft + drgt);
-    dsgn = copysign(R(1), dcen);
     dlim = (dlft * drgt >= R(0)) ? R(2) * dmin(fabs(dlft), fabs(drgt)) : R(0);
-    dfm = dsgn * dmin(dlim, fabs(dcen));
+    dfm = copysign(dmin(dlim, fabs(dcen)), dcen);
     dlft = qp - qc;
     drgt = qp2 - qp;
     dcen = R(0.5) * (dlft + drgt);
-    dsgn = copysign(R(1), dcen);
     dlim = (dlft * drgt >= R(0)) ? R(2) * dmin(fabs(dlft), fabs(drgt)) : R(0);
-    dfp = dsgn * dmin(dlim, fabs(dcen));
+    dfp = copysign(dmin(dlim, fabs(dcen)), dcen);
   }
   dlft = qc - qm;
   drgt = qp - qc;
   dcen = R(0.5) * (dlft + drgt);
-  dsgn = copysign(R(1), dcen);
   dlim = (dlft * drgt >= R(0)) ? R(2) * dmin(fabs(dlft), fabs(drgt)) : R(0);
   dtemp = (order == 2) ? dcen : R(4) / R(3) * dcen - R(1) / R(6) * (dfp + dfm);
-  return flat * dsgn * dmin(dlim, fabs(dtemp));
+  return copysign(flat, dcen) * dmin(dlim, fabs(dtemp));  // flat is not negative
 }
 
 // ------------------------------------------------------------------ Riemann

@@ -494,12 +494,12 @@ __device__ __forceinline__ void trace_ppm_dir(const pcg::Region& rg, const PT& P
   R sm, sp, sc, s6;
   R Imr[3], Ipr[3], Imu[3], Ipu[3], Imp[3], Ipp[3];
   R Imt[3], Ipt[3];
-  const R sp3[3] = {un - cc, un, un + cc};
+  const PpmWave<R> wv[3] = {ppm_wave_of<R>(un - cc, dtdx), ppm_wave_of<R>(un, dtdx), ppm_wave_of<R>(un + cc, dtdx)};
   const R p0 = R(p0_of<NS, MIX, R>(rg));
 #define PROFILE3(comp, Im, Ip)                                      \
   ppm_edges<HYB, R>(P, comp, flat, scheme, sm, sp, sc);              \
   s6 = ppm_s6<R>(sm, sp, sc);                                        \
-  _Pragma("unroll") for (int w = 0; w < 3; ++w) ppm_wave<R>(sm, sp, s6, sp3[w], dtdx, Ip[w], Im[w]);
+  _Pragma("unroll") for (int w = 0; w < 3; ++w) ppm_wave<R>(sm, sp, s6, wv[w], Ip[w], Im[w]);
   PROFILE3(pcg::QRHO, Imr, Ipr)
   PROFILE3(pcg::QU + D, Imu, Ipu)
   PROFILE3(pcg::QPRES, Imp, Ipp)
@@ -508,7 +508,7 @@ __device__ __forceinline__ void trace_ppm_dir(const pcg::Region& rg, const PT& P
     if (c == D) continue;
     ppm_edges<HYB, R>(P, pcg::QU + c, flat, scheme, sm, sp, sc);
     s6 = ppm_s6<R>(sm, sp, sc);
-    ppm_wave<R>(sm, sp, s6, un, dtdx, Ipt[c], Imt[c]);
+    ppm_wave<R>(sm, sp, s6, wv[1], Ipt[c], Imt[c]);
   }
   R ym0[NS], ym1[NS], yp1[NS], yp2[NS];
   if constexpr (SLOTS) {
@@ -527,7 +527,7 @@ __device__ __forceinline__ void trace_ppm_dir(const pcg::Region& rg, const PT& P
       }
       s6 = ppm_s6<R>(sm, sp, sc);
 #pragma unroll
-      for (int w = 0; w < 3; ++w) ppm_wave<R>(sm, sp, s6, sp3[w], dtdx, Ip[w], Im[w]);
+      for (int w = 0; w < 3; ++w) ppm_wave<R>(sm, sp, s6, wv[w], Ip[w], Im[w]);
       R* y = slots + 4 * 128 * n;
       y[0] = Im[0];
       y[128] = Im[1];
