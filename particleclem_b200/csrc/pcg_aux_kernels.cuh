@@ -318,9 +318,9 @@ static cudaError_t launch_advance_t(const pcg::StageArgs& a, int64_t nblocks, in
   if (nblocks <= 0) return cudaSuccess;
   const unsigned grid = (unsigned)nblocks;
   switch (variant) {
-    case 0: return launch_kernel(k_advance<NS, MIX, kMinBlocks[K_CONSUP][0]>, grid, a, s);
-    case 1: return launch_kernel(k_advance<NS, MIX, kMinBlocks[K_CONSUP][1]>, grid, a, s);
-    case 2: return launch_kernel(k_advance<NS, MIX, kMinBlocks[K_CONSUP][2]>, grid, a, s);
+    case 0: return launch_kernel(k_advance<NS, MIX, min_blocks<NS>(K_CONSUP, 0)>, grid, a, s);
+    case 1: return launch_kernel(k_advance<NS, MIX, min_blocks<NS>(K_CONSUP, 1)>, grid, a, s);
+    case 2: return launch_kernel(k_advance<NS, MIX, min_blocks<NS>(K_CONSUP, 2)>, grid, a, s);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -35,15 +35,15 @@ constexpr bool kExact = false;  // reduced algebra
 template <int NS, bool MIX, class R, int V>
 static cudaError_t launch_v(int stage, const pcg::StageArgs& a, unsigned grid, cudaStream_t s) {
   switch (stage) {
-    case K_CTOPRIM: return launch_kernel(k_ctoprim<NS, MIX, kMinBlocks[K_CTOPRIM][V]>, grid, a, s);
+    case K_CTOPRIM: return launch_kernel(k_ctoprim<NS, MIX, min_blocks<NS>(K_CTOPRIM, V)>, grid, a, s);
     case K_PREP: return launch_kernel(k_prep<NS, MIX, kExact, R>, grid, a, s);
     case K_TRACE:
       if (a.use_hybrid_weno && a.ppm_type == 1)
         return launch_kernel(k_trace_weno<NS, MIX, kExact, R>, grid, a, s);  // one shape for every variant
-      return launch_kernel(k_trace<NS, MIX, kExact, R, kMinBlocks[K_TRACE][V]>, grid, a, s);
-    case K_FLUX0: return launch_kernel(k_flux0<NS, MIX, kExact, R, kMinBlocks[K_FLUX0][V]>, grid, a, s);
-    case K_FLUX1: return launch_kernel(k_flux1<NS, MIX, kExact, R, kMinBlocks[K_FLUX1][V]>, grid, a, s);
-    case K_FLUX2: return launch_kernel(k_flux2<NS, MIX, kExact, R, kMinBlocks[K_FLUX2][V]>, grid, a, s);
+      return launch_kernel(k_trace<NS, MIX, kExact, R, min_blocks<NS>(K_TRACE, V)>, grid, a, s);
+    case K_FLUX0: return launch_kernel(k_flux0<NS, MIX, kExact, R, min_blocks<NS>(K_FLUX0, V)>, grid, a, s);
+    case K_FLUX1: return launch_kernel(k_flux1<NS, MIX, kExact, R, min_blocks<NS>(K_FLUX1, V)>, grid, a, s);
+    case K_FLUX2: return launch_kernel(k_flux2<NS, MIX, kExact, R, min_blocks<NS>(K_FLUX2, V)>, grid, a, s);
     case K_CONSUP: return launch_kernel(k_consup<NS, MIX>, grid, a, s);
     case K_LOWBC: return launch_kernel(k_lowbc<NS, MIX, kExact, R>, grid, a, s);
     default: return cudaErrorInvalidValue;
@@ -69,9 +69,9 @@ static cudaError_t launch_trace_tile(const pcg::StageArgs& a, unsigned grid, int
                                     cudaStream_t s) {
   if constexpr (sizeof(R) == 4 && pcg::trace_tile_species(NS)) {
     switch (variant) {
-      case 0: return launch_kernel(k_trace_tile<NS, MIX, kMinBlocks[K_TRACE][0]>, grid, a, s);
-      case 1: return launch_kernel(k_trace_tile<NS, MIX, kMinBlocks[K_TRACE][1]>, grid, a, s);
-      case 2: return launch_kernel(k_trace_tile<NS, MIX, kMinBlocks[K_TRACE][2]>, grid, a, s);
+      case 0: return launch_kernel(k_trace_tile<NS, MIX, min_blocks<NS>(K_TRACE, 0)>, grid, a, s);
+      case 1: return launch_kernel(k_trace_tile<NS, MIX, min_blocks<NS>(K_TRACE, 1)>, grid, a, s);
+      case 2: return launch_kernel(k_trace_tile<NS, MIX, min_blocks<NS>(K_TRACE, 2)>, grid, a, s);
       default: return cudaErrorInvalidValue;
     }
   } else {

@@ -125,22 +125,24 @@ constexpr size_t kAlign = 256;
 
 thread_local std::string g_err;
 
-// Launch-variant table: [precision_mode][species slot][stage] -> variant index of
+// Launch-variant table: [precision_mode][species class][stage] -> variant index of
 // kMinBlocks (pcg_kernels.cuh). Defaults measured on B200 for the production flame
 // level; pcg_set_launch_variant (the autotuner) overrides them. The mixed form's trace
 // has three more variants: 3-5 run the TMA-staged tiled trace (K_TRACE_TILE) with the
 // register budgets 0-2.
 constexpr int kTileVariant = 3;
 std::mutex g_var_mu;
-int g_variant[3][2][7] = {
-  {{0, 0, 2, 0, 1, 2, 1}, {2, 0, 2, 1, 0, 0, 2}},  // FP64 reference order
-  {{1, 0, 1, 0, 0, 0, 1}, {2, 0, 2, 0, 0, 0, 1}},  // FP64 with FMA
-  {{0, 0, 2, 0, 1, 0, 1}, {2, 0, 0, 0, 0, 2, 2}},  // mixed
+int g_variant[3][3][7] = {
+  // one species, 2 to 12 species, more (whose kernels spill under every cap)
+  {{0, 0, 2, 0, 2, 2, 2}, {2, 0, 2, 1, 0, 0, 2}, {1, 0, 0, 0, 0, 0, 1}},  // FP64 reference order
+  {{1, 0, 1, 0, 0, 0, 1}, {2, 0, 2, 0, 1, 0, 1}, {1, 0, 0, 0, 0, 0, 1}},  // FP64 with FMA
+  {{2, 0, 2, 0, 1, 2, 2}, {2, 0, 0, 0, 1, 2, 2}, {1, 0, 0, 0, 1, 0, 1}},  // mixed
 };
+int species_class(int ns) { return ns == 1 ? 0 : ns <= 12 ? 1 : 2; }
 int max_variant(int prec, int stage) { return (prec == PCG_PREC_MIXED && stage == K_TRACE) ? 5 : 2; }
 int variant_of(int prec, int ns, int stage) {
   std::lock_guard<std::mutex> lk(g_var_mu);
-  return g_variant[prec][ns == 1 ? 0 : 1][stage];
+  return g_variant[prec][species_class(ns)][stage];
 }
 
 // Stream-ordered workspace pool per device. Its release threshold is unbounded, so
@@ -458,7 +460,9 @@ void add_seg(Layout& L, int stage, int region, int variant, const IBox& b) {
 // direction segments (kOrderRegionBytes) the k_flux2 direction segments are therefore
 // interleaved in slabs of kOrderSlab z-planes (x, y, z of one slab, then the next slab)
 // so that a slab's state comes from DRAM once. Measured on the 128^3 flame level (mixed
-// form): flux2 0.672 -> 0.657 ms. The same interleave slowed the stages whose
+// form): flux2 0.672 -> 0.657 ms, later 0.628 -> 0.616. With one species the state is a smaller
+// part of what flux2 reads and the three directions' code competes for the instruction caches
+// (256^3, mixed: 2.35 -> 2.49 ms), so one-species regions keep whole directions. The same interleave slowed the stages whose
 // directions run different code (flux1 0.661 -> 0.726 ms, trace 0.631 -> 0.658, flux0
 // 0.228 -> 0.245), so they keep one segment per direction (PCG_ORDER_SLABS: bit K_* of
 // the stages that interleave).
@@ -643,7 +647,7 @@ void build_layout(Layout& L, const std::vector<BoxIn>& boxes, const pcg_hydro_pa
     R.zero_uout = B.zero_uout ? 1 : 0;
     const IBox g4 = grow(B.bx, 4), g1 = grow(B.bx, 1);
     // direction segments interleaved in z-slabs for large regions (see add_dir_segs)
-    const bool slabs = g1.cells() * nv * 8 > kOrderRegionBytes && B.bx.n(2) >= 2 * kOrderSlab;
+    const bool slabs = ns > 1 && g1.cells() * nv * 8 > kOrderRegionBytes && B.bx.n(2) >= 2 * kOrderSlab;
     const int z0 = B.bx.lo[2];
     IBox sb[3];
     if (B.internal_q) {
@@ -1916,7 +1920,7 @@ int pcg_set_launch_variant(int32_t precision_mode, int32_t nspec, int32_t stage,
       variant < 0 || variant > max_variant(precision_mode, stage))
     return fail(PCG_EINVAL, "launch variant (%d, %d, %d, %d) out of range", precision_mode, nspec, stage, variant);
   std::lock_guard<std::mutex> lk(g_var_mu);
-  g_variant[precision_mode][nspec == 1 ? 0 : 1][stage] = variant;
+  g_variant[precision_mode][species_class(nspec)][stage] = variant;
   return PCG_OK;
 }
 

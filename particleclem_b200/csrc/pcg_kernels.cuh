@@ -36,16 +36,32 @@ enum { K_LOWBC = K_NSTAGE, K_SRCQ, K_TRACE_TILE };
 
 // Launch variants: each heavy stage is compiled with a few minimum-resident-blocks
 // requests (__launch_bounds__ register caps); the host picks one per (form, species
-// count, stage) from a table the autotuner fills. 0 = no cap.
-constexpr int kMinBlocks[K_NSTAGE][3] = {
-  {0, 5, 8},  // ctoprim
-  {0, 0, 0},  // prep
-  {0, 4, 5},  // trace
-  {0, 6, 8},  // flux0
-  {5, 6, 8},  // flux1
-  {4, 5, 6},  // flux2
-  {0, 5, 6},  // consup: the caps apply to the fused step tail (k_advance)
+// class, stage) from a table the autotuner fills. 0 = no cap. One species needs fewer
+// registers, so its kernels gain from tighter caps (256^3, mixed form: flux2 2.75 ms at 6 blocks,
+// 2.38 at 8; trace 2.07 at 5, 1.92 at 8; ctoprim 0.39 uncapped, 0.35 at 12).
+constexpr int kMinBlocks[2][K_NSTAGE][3] = {
+  {
+    // one species
+    {0, 5, 12},  // ctoprim
+    {0, 0, 0},   // prep
+    {0, 6, 8},   // trace
+    {0, 6, 8},   // flux0
+    {5, 6, 8},   // flux1
+    {4, 6, 8},   // flux2
+    {0, 5, 8},   // consup: the caps apply to the fused step tail (k_advance)
+  },
+  {
+    // mixtures
+    {0, 5, 8},  // ctoprim
+    {0, 0, 0},  // prep
+    {0, 4, 5},  // trace
+    {0, 5, 8},  // flux0
+    {4, 5, 8},  // flux1
+    {4, 5, 6},  // flux2
+    {0, 5, 6},  // consup
+  },
 };
+template <int NS> constexpr int min_blocks(int stage, int variant) { return kMinBlocks[NS == 1 ? 0 : 1][stage][variant]; }
 
 struct Item {
   const pcg::Region* rg;
