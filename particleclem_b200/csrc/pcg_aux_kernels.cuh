@@ -41,16 +41,7 @@ __device__ __forceinline__ double block_min(double v) {
 
 // Source/Timestep.H:51-88 (pc_estdt_hydro) for one cell of state s:
 // min over d of dx_d / (c + |u_d|), c from the stored temperature.
-template <int NS, bool MIX>
-__device__ __forceinline__ double cfl_dt(const double* s, const double* dx) {
-  using E = Eos<NS, MIX, double>;
-  const double rho = s[pcg::URHO];
-  const double rhoInv = 1.0 / rho;
-  const double T = s[pcg::UTEMP];
-  double y[NS];
-#pragma unroll
-  for (int n = 0; n < NS; ++n) y[n] = s[pcg::UFS + n] * rhoInv;
-  const double c = E::rty2cs(rho, T, y);
+__device__ __forceinline__ double cfl_of(const double* s, const double* dx, double rhoInv, double c) {
   double dt = DBL_MAX;
   const double ux = s[pcg::UMX] * rhoInv;
   dt = dmin(dt, dx[0] / (c + fabs(ux)));
@@ -59,6 +50,16 @@ __device__ __forceinline__ double cfl_dt(const double* s, const double* dx) {
   const double uz = s[pcg::UMZ] * rhoInv;
   dt = dmin(dt, dx[2] / (c + fabs(uz)));
   return dt;
+}
+template <int NS, bool MIX>
+__device__ __forceinline__ double cfl_dt(const double* s, const double* dx) {
+  using E = Eos<NS, MIX, double>;
+  const double rho = s[pcg::URHO];
+  const double rhoInv = 1.0 / rho;
+  double y[NS];
+#pragma unroll
+  for (int n = 0; n < NS; ++n) y[n] = s[pcg::UFS + n] * rhoInv;
+  return cfl_of(s, dx, rhoInv, E::rty2cs(rho, s[pcg::UTEMP], y));
 }
 
 // Per-cell CFL constraints of every valid cell, block minima.
@@ -121,9 +122,9 @@ __global__ void __launch_bounds__(kFinalThreads) k_estdt_final(const __grid_cons
 // (PeleCUtilities.H:70-84), on one cell: s holds S_old on entry and S_new on exit.
 // construct_Snew's pc_rst_int_e and computeTemp on the state s (already S_old + dt *
 // hydro source).
-template <int NS, bool MIX>
-__device__ __forceinline__ void finish_cell(double* s) {
-  using E = Eos<NS, MIX, double>;
+// The internal energy of S_new into s (pc_rst_int_e), its mass fractions into y; returns e.
+template <int NS>
+__device__ __forceinline__ double energy_cell(double* s, double* y) {
   const double rho = s[pcg::URHO];
   const double rhoInv = 1.0 / rho;
   const double Up = s[pcg::UMX] * rhoInv;
@@ -133,10 +134,32 @@ __device__ __forceinline__ void finish_cell(double* s) {
   s[pcg::UEINT] = s[pcg::UEDEN] - rho * ke;
   const double rhoInv2 = 1.0 / s[pcg::URHO];
   const double e = s[pcg::UEINT] * rhoInv2;
-  double y[NS];
 #pragma unroll
   for (int n = 0; n < NS; ++n) y[n] = s[pcg::UFS + n] * rhoInv2;
+  return e;
+}
+template <int NS, bool MIX>
+__device__ __forceinline__ void finish_cell(double* s) {
+  using E = Eos<NS, MIX, double>;
+  double y[NS];
+  const double e = energy_cell<NS>(s, y);
   s[pcg::UTEMP] = E::rey2t(e, y, s[pcg::UTEMP]);
+}
+// finish_cell and the CFL constraint of the result in one, sharing the mixture polynomial.
+template <int NS, bool MIX>
+__device__ __forceinline__ double finish_cfl(double* s, const double* dx) {
+  if (MIX && !kExact && EosC<double, MIX>::uniform_tmid()) {
+    double y[NS];
+    const double e = energy_cell<NS>(s, y);
+    const double rm = Eos<NS, MIX, double>::rmix(y);
+    MixPoly<NS> mp;
+    const double T = mp.temperature(e, y, s[pcg::UTEMP]);
+    s[pcg::UTEMP] = T;
+    const double rho = s[pcg::URHO], cv = mp.cv(T), p = rho * rm * T, g = (cv + rm) / cv;
+    return cfl_of(s, dx, 1.0 / rho, sqrt(g * p / rho));
+  }
+  finish_cell<NS, MIX>(s);
+  return cfl_dt<NS, MIX>(s, dx);
 }
 
 template <int NS, bool MIX>
@@ -188,10 +211,9 @@ __global__ void __launch_bounds__(128, MINB) k_advance(const __grid_constant__ p
       consup_each<NS, float>(rg, it.i, it.j, it.k, p0_of<NS, MIX, float>(rg), add);
     else
       consup_each<NS, double>(rg, it.i, it.j, it.k, 0.0, add);
-    finish_cell<NS, MIX>(s);
+    dtc = finish_cfl<NS, MIX>(s, rg.dx);
 #pragma unroll
     for (int n = 0; n < pcg::nvar(NS); ++n) u[n] = s[n];
-    dtc = cfl_dt<NS, MIX>(s, rg.dx);
   }
   dtc = block_min(dtc);
   if (threadIdx.x == 0) a.partial[blockIdx.x] = dtc;

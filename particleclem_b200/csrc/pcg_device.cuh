@@ -14,6 +14,12 @@
 
 namespace PCG_TU {
 
+#ifdef PCG_TU_DOUBLE_ONLY
+constexpr bool kExact = true;  // reference expression order
+#else
+constexpr bool kExact = false;  // reduced algebra
+#endif
+
 // ------------------------------------------------------------------ constants
 template <class R> struct Lim;
 template <> struct Lim<double> {
@@ -486,6 +492,54 @@ struct EosR {
     if (!MIX) return p * rrcp(C::gamma() - R(1));
     const R t = rdiv(p, eos_ru<R>() * sum_imw(w));
     return E::e_of(t, w);
+  }
+};
+
+// The mixture's energy polynomial at a fixed composition, e(T) = sum_i a_i T^i with a_i =
+// sum_k Y_k ec[k][range][i]; its derivative is cv (the species tables satisfy cv_k = de_k/dT).
+// The Newton solve for T then costs 9 operations per iteration and NS * 6 once, where the
+// species sums cost NS * 11 per iteration, and the mass fractions are dead once the
+// coefficients and rmix exist. FP64 step tail and ctoprim of the reduced forms, with one range
+// switch temperature for all species (tables with several take the species sums).
+template <int NS>
+struct MixPoly {
+  using C = EosC<double, true>;
+  double a[6];
+  int range;
+  template <int RG>
+  __device__ __forceinline__ void sum(const double* y) {
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+      double v = 0.0;
+#pragma unroll
+      for (int k = 0; k < NS; ++k) v = v + y[k] * C::ecr(k, RG, i);
+      a[i] = v;
+    }
+  }
+  __device__ __forceinline__ void set(const double* y, double t) {
+    range = t < C::tmid(0) ? 0 : 1;
+    if (range == 0) sum<0>(y); else sum<1>(y);
+  }
+  __device__ __forceinline__ bool holds(double t) const { return (t < C::tmid(0) ? 0 : 1) == range; }
+  __device__ __forceinline__ double e(double t) const {
+    return a[0] + t * (a[1] + t * (a[2] + t * (a[3] + t * (a[4] + t * a[5]))));
+  }
+  __device__ __forceinline__ double cv(double t) const {
+    return a[1] + t * (2.0 * a[2] + t * (3.0 * a[3] + t * (4.0 * a[4] + t * (5.0 * a[5]))));
+  }
+  // Eos::rey2t; leaves the polynomial of the result's range
+  __device__ __forceinline__ double temperature(double en, const double* y, double tguess) {
+    double tt = tguess;
+    if (!(tt > 0.0)) tt = 1000.0;
+    set(y, tt);
+    for (int it = 0; it < pcg::NEWTON_MAXIT; ++it) {
+      const double dt = (en - e(tt)) / cv(tt);
+      tt = tt + dt;
+      if (tt < pcg::NEWTON_TMIN) tt = pcg::NEWTON_TMIN;
+      if (!holds(tt)) set(y, tt);
+      if (fabs(dt) <= pcg::NEWTON_RTOL * tt) break;
+    }
+    return tt;
   }
 };
 

@@ -26,12 +26,6 @@ cudaError_t upload_eos(int slot, const pcg::EosConst& e) {
   return cudaMemcpyToSymbol(c_eos, &e, sizeof(e), slot * sizeof(e), cudaMemcpyHostToDevice);
 }
 
-#ifdef PCG_TU_DOUBLE_ONLY
-constexpr bool kExact = true;  // reference expression order
-#else
-constexpr bool kExact = false;  // reduced algebra
-#endif
-
 template <int NS, bool MIX, class R, int V>
 static cudaError_t launch_v(int stage, const pcg::StageArgs& a, unsigned grid, cudaStream_t s) {
   switch (stage) {
