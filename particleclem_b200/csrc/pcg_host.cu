@@ -134,9 +134,9 @@ constexpr int kTileVariant = 3;
 std::mutex g_var_mu;
 int g_variant[3][3][7] = {
   // one species, 2 to 12 species, more (whose kernels spill under every cap)
-  {{0, 0, 2, 0, 2, 2, 2}, {2, 0, 2, 1, 0, 0, 2}, {1, 0, 0, 0, 0, 0, 1}},  // FP64 reference order
-  {{1, 0, 1, 0, 0, 0, 1}, {2, 0, 2, 0, 1, 0, 1}, {1, 0, 0, 0, 0, 0, 1}},  // FP64 with FMA
-  {{2, 0, 2, 0, 1, 2, 2}, {2, 0, 0, 0, 1, 2, 2}, {1, 0, 0, 0, 1, 0, 1}},  // mixed
+  {{0, 0, 2, 0, 2, 1, 2}, {2, 0, 2, 1, 1, 0, 2}, {1, 0, 0, 0, 0, 0, 1}},  // FP64 reference order
+  {{0, 0, 2, 0, 0, 0, 0}, {2, 0, 2, 1, 0, 0, 0}, {1, 0, 0, 0, 0, 0, 1}},  // FP64 with FMA
+  {{2, 0, 2, 0, 1, 2, 2}, {2, 0, 0, 0, 1, 2, 2}, {1, 0, 0, 1, 0, 0, 1}},  // mixed
 };
 int species_class(int ns) { return ns == 1 ? 0 : ns <= 12 ? 1 : 2; }
 int max_variant(int prec, int stage) { return (prec == PCG_PREC_MIXED && stage == K_TRACE) ? 5 : 2; }
@@ -879,15 +879,21 @@ void set_segs(A& a, const std::vector<pcg::Seg>& v) {
 // (more) it, where those are the library's own in the same call. It saves the launch gap, a
 // few microseconds per launch, and costs each block about 0.3 us at its start (traces of
 // 17000 and 51000 blocks ran 3-5 % longer with it), so launches of many waves go without.
-// In a captured graph, whose launches have no such gap, the step of a 32^3 level took 53.9 us
-// without and 57.2 us with it (16^3, 9 species, FP64: 106 and 121 us): none there.
 constexpr int64_t kOverlapBlocks = 4096;
-int overlap_launch(int64_t nblocks, bool after, bool more, cudaStream_t s) {
+int overlap_launch(int64_t nblocks, bool after, bool more) {
   if (nblocks > kOverlapBlocks) return 0;
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) cudaGetLastError();
-  if (cs != cudaStreamCaptureStatusNone) return 0;
   return (after ? pcg::kOverlapPrevious : 0) | (more ? pcg::kOverlapNext : 0);
+}
+// Whether a call's launches may overlap at all: not in a captured graph, whose launches have
+// no such gap (step of a 32^3 level 53.9 us without overlap, 57.2 us with it; 16^3, 9 species,
+// FP64: 106 and 121 us; one 16^3 box of one species, launched on a stream: 74 and 66 us).
+bool may_overlap(cudaStream_t s) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return cs == cudaStreamCaptureStatusNone;
 }
 
 // One launch of the kernel of `stage` over the segments of kind `segs` (launch variant var).
@@ -907,7 +913,7 @@ int launch_segs(const Layout& L, const Tables& T, const pcg_hydro_params* p, int
   a.use_hybrid_weno = p->use_hybrid_weno;
   a.weno_scheme = p->weno_scheme;
   a.umeth = L.umeth;
-  a.overlap = overlap_launch(L.nblocks[segs], after, more, s);
+  a.overlap = overlap_launch(L.nblocks[segs], after, more);
   a.difmag = p->difmag;
   a.dt_dev = dt_dev;
   cudaError_t e = (p->precision_mode == PCG_PREC_FP64)
@@ -931,10 +937,11 @@ int launch_kind(const Layout& L, const Tables& T, const pcg_hydro_params* p, int
 // after, more: the call has launches of its own before the first stage, behind the last.
 int launch_stages(const Layout& L, const Tables& T, const pcg_hydro_params* p, int first, int last,
                   const double* dt_dev, cudaStream_t s, bool after = false, bool more = false) {
+  const bool live = may_overlap(s);
   for (int st = first; st <= last; ++st) {
-    const bool next = st < last || more;
-    int rc = launch_kind(L, T, p, st, dt_dev, after || st > first, next, s);
-    if (rc == PCG_OK && st == K_FLUX2) rc = launch_kind(L, T, p, K_LOWBC, dt_dev, true, next, s);
+    const bool next = live && (st < last || more);
+    int rc = launch_kind(L, T, p, st, dt_dev, live && (after || st > first), next, s);
+    if (rc == PCG_OK && st == K_FLUX2) rc = launch_kind(L, T, p, K_LOWBC, dt_dev, live, next, s);
     if (rc) return rc;
   }
   return PCG_OK;
@@ -1487,14 +1494,14 @@ int pcg_step_boxes(const pcg_hydro_params* prm, int32_t nbox, const pcg_box* box
   }
   bind_tables(T2);
   double* partial = reinterpret_cast<double*>(base + off_p);
-  const bool strict = prm->precision_mode == PCG_PREC_FP64;
+  const bool strict = prm->precision_mode == PCG_PREC_FP64, live = may_overlap(s);
   if (fill_ghosts) {
     pcg::AuxArgs f{};
     f.fills = reinterpret_cast<const pcg::FillBox*>(base + off_f);
     f.nfill = nbox;
     f.ng = 4;
     f.ncomp = nv;
-    f.overlap = overlap_launch(fill_blocks, false, true, s);
+    f.overlap = overlap_launch(fill_blocks, false, live);
     e = pcg_strict::launch_aux(AUX_FILL_BOXES, prm->nspec, f, fill_blocks, s);
     if (e != cudaSuccess) rc = fail(PCG_ECUDA, "ghost fill: %s", cudaGetErrorString(e));
   }
@@ -1505,7 +1512,7 @@ int pcg_step_boxes(const pcg_hydro_params* prm, int32_t nbox, const pcg_box* box
     a.segs = T2.segs[K_CONSUP];
     set_segs(a, L.segs[K_CONSUP]);
     a.partial = partial;
-    a.overlap = overlap_launch(L.nblocks[K_CONSUP], true, true, s);
+    a.overlap = overlap_launch(L.nblocks[K_CONSUP], live, live);
     const int v = variant_of(prm->precision_mode, prm->nspec, K_CONSUP);
     e = strict ? pcg_strict::launch_advance(prm->nspec, a, L.nblocks[K_CONSUP], v, s)
                : pcg_fast::launch_advance(prm->nspec, a, L.nblocks[K_CONSUP], v, s);
@@ -1515,7 +1522,7 @@ int pcg_step_boxes(const pcg_hydro_params* prm, int32_t nbox, const pcg_box* box
       r.partial = partial;
       r.cfl = cfl;
       r.dt_boxes = dt_next;
-      r.overlap = overlap_launch(nbox, true, false, s);
+      r.overlap = overlap_launch(nbox, live, false);
       e = pcg_strict::launch_aux(AUX_ESTDT_BOXES, prm->nspec, r, nbox, s);
     }
     if (e != cudaSuccess) rc = fail(PCG_ECUDA, "step tail: %s", cudaGetErrorString(e));
@@ -1581,9 +1588,10 @@ int pcg_estdt(int32_t nspec, int32_t nbox, const pcg_box* boxes, double cfl, dou
     a.npartial = nblocks;
     a.cfl = cfl;
     a.dt_out = dt_out;
-    a.overlap = overlap_launch(nblocks, false, true, s);
+    const bool live = may_overlap(s);
+    a.overlap = overlap_launch(nblocks, false, live);
     e = pcg_strict::launch_aux(AUX_ESTDT, nspec, a, nblocks, s);
-    a.overlap = overlap_launch(1, true, false, s);
+    a.overlap = overlap_launch(1, live, false);
     if (e == cudaSuccess) e = pcg_strict::launch_aux(AUX_ESTDT_FINAL, nspec, a, 1, s);
   }
   if (e != cudaSuccess) rc = fail(PCG_ECUDA, "estdt: %s", cudaGetErrorString(e));
@@ -1828,9 +1836,10 @@ int pcg_plan_estdt(pcg_plan* P, double cfl, double* dt_dev, pcg_stream_t stream)
   a.cfl = cfl;
   a.dt_out = dt_dev;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  a.overlap = overlap_launch(P->aux_blocks, false, true, s);
+  const bool live = may_overlap(s);
+  a.overlap = overlap_launch(P->aux_blocks, false, live);
   cudaError_t e = pcg_strict::launch_aux(AUX_ESTDT, P->prm.nspec, a, P->aux_blocks, s);
-  a.overlap = overlap_launch(1, true, false, s);
+  a.overlap = overlap_launch(1, live, false);
   if (e == cudaSuccess) e = pcg_strict::launch_aux(AUX_ESTDT_FINAL, P->prm.nspec, a, 1, s);
   return e == cudaSuccess ? PCG_OK : fail(PCG_ECUDA, "estdt: %s", cudaGetErrorString(e));
 }
@@ -1867,7 +1876,8 @@ int pcg_plan_advance(pcg_plan* P, double cfl, const double* dt_dev, double* dt_n
   // few blocks: the last one takes their minimum itself, which saves a launch; of many, the
   // cluster of k_estdt_final does it sooner
   const bool one_launch = nb <= kTailBlocks;
-  a.overlap = overlap_launch(nb, true, !one_launch, s);
+  const bool live = may_overlap(s);
+  a.overlap = overlap_launch(nb, live, live && !one_launch);
   if (one_launch) {
     a.done = P->d_done;
     a.cfl = cfl;
@@ -1882,7 +1892,7 @@ int pcg_plan_advance(pcg_plan* P, double cfl, const double* dt_dev, double* dt_n
     f.npartial = nb;
     f.cfl = cfl;
     f.dt_out = dt_next;
-    f.overlap = overlap_launch(1, true, false, s);
+    f.overlap = overlap_launch(1, live, false);
     e = pcg_strict::launch_aux(AUX_ESTDT_FINAL, P->prm.nspec, f, 1, s);
   }
   return e == cudaSuccess ? PCG_OK : fail(PCG_ECUDA, "advance: %s", cudaGetErrorString(e));
