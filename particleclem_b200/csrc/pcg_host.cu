@@ -1161,32 +1161,32 @@ namespace {
 // Whether cv of the polynomial c (5 coefficients) is positive on [t, t + h], by more than
 // FP32 rounding of its terms: its value at t against the largest change over h.
 bool cv_positive(const double* c, double t, double h) {
-  double v = 0.0, mag = 0.0, slope = 0.0, p = 1.0;
+  double v = 0.0, mag = 0.0, slope = 0.0;
   const double te = t + h;
-  for (int i = 0; i < 5; ++i) {
-    v += c[i] * p;
-    p *= t;
-    mag += std::fabs(c[i]) * std::pow(te, i);
-    if (i) slope += std::fabs(c[i]) * i * std::pow(te, i - 1);
+  for (int i = 4; i >= 0; --i) {
+    slope = slope * te + mag;  // derivative of mag, the sum of |terms| at te
+    mag = mag * te + std::fabs(c[i]);
+    v = v * t + c[i];
   }
   return v - slope * h > 1e-4 * mag;
 }
 
 // EosConst::star_lo/hi of a mixture table: the widest temperature range around the
-// species' range switches (scanned in 1 K steps, up to 20000 K) in which every cv_k is
-// positive, as bounds on p / rho = RU T sum(Y / W) that hold for any composition.
+// species' range switches (scanned in steps of kScanStep, up to kScanTop) in which every cv_k
+// is positive, as bounds on p / rho = RU T sum(Y / W) that hold for any composition.
+constexpr double kScanStep = 20.0, kScanTop = 20000.0;
 void star_bounds(pcg::EosConst& c) {
-  double lo = 0.0, hi = 20000.0, wmin = 1.0 / c.imw[0], wmax = wmin;
+  double lo = 0.0, hi = kScanTop, wmin = 1.0 / c.imw[0], wmax = wmin;
   for (int k = 0; k < c.nspec; ++k) {
     wmin = std::min(wmin, 1.0 / c.imw[k]);
     wmax = std::max(wmax, 1.0 / c.imw[k]);
     // the switch clamped to the scanned range (a NaN switch always takes the upper range)
-    const double tm = c.tmid[k] > 0.0 ? std::min(c.tmid[k], 20000.0) : 0.0;
+    const double tm = c.tmid[k] > 0.0 ? std::min(c.tmid[k], kScanTop) : 0.0;
     double t = tm;
-    while (t < hi && cv_positive(c.cvc[k][1], t, 1.0)) t += 1.0;
+    while (t < hi && cv_positive(c.cvc[k][1], t, kScanStep)) t += kScanStep;
     hi = std::min(hi, t);
     t = tm;
-    while (t > lo && cv_positive(c.cvc[k][0], std::max(t - 1.0, 0.0), 1.0)) t -= 1.0;
+    while (t > lo && cv_positive(c.cvc[k][0], std::max(t - kScanStep, 0.0), kScanStep)) t -= kScanStep;
     lo = std::max(lo, t);
   }
   lo = std::max(lo, 1e-3);
