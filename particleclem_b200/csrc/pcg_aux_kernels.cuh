@@ -217,19 +217,6 @@ __global__ void __launch_bounds__(128, MINB) k_advance(const __grid_constant__ p
   }
   dtc = block_min(dtc);
   if (threadIdx.x == 0) a.partial[blockIdx.x] = dtc;
-  if (!a.done) return;
-  __shared__ bool last;
-  if (threadIdx.x == 0) {
-    __threadfence();  // the block's minimum before its count
-    last = atomicInc(a.done, gridDim.x - 1) == gridDim.x - 1;
-    __threadfence();
-  }
-  __syncthreads();
-  if (!last) return;
-  double v = DBL_MAX;
-  for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) v = dmin(v, __ldcg(a.partial + b));
-  v = block_min(v);
-  if (threadIdx.x == 0) *a.dt_out = v * a.cfl;
 }
 
 // Single-level FillBoundary of a domain FAB that covers grow(domain, ng), every ghost

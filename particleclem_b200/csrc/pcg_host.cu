@@ -1108,11 +1108,10 @@ struct pcg_plan {
   std::vector<pcg::AuxBox> aux;
   std::vector<pcg::Seg> aux_segs;
   int64_t aux_blocks = 0;
-  void* aux_dev = nullptr;  // AuxBox[] + Seg[] + partial[] + done
+  void* aux_dev = nullptr;  // AuxBox[] + Seg[] + partial[]
   pcg::AuxBox* d_aux = nullptr;
   pcg::Seg* d_aux_segs = nullptr;
   double* d_partial = nullptr;
-  unsigned* d_done = nullptr;  // blocks of the step tail that have finished (zero between steps)
   int device = 0;
 };
 
@@ -1783,7 +1782,7 @@ int pcg_plan_create(const pcg_hydro_params* prm, int32_t nbox, const pcg_box* bo
                b3 = std::max<int64_t>(P->aux_blocks, P->L.nblocks[K_CONSUP]) * sizeof(double);
   if ((e = cudaMalloc(&P->T.dev, P->T.bytes)) == cudaSuccess &&
       (e = cudaMemcpy(P->T.dev, P->T.host.data(), P->T.bytes, cudaMemcpyHostToDevice)) == cudaSuccess &&
-      (e = cudaMalloc(&P->aux_dev, b1 + b2 + b3 + sizeof(unsigned))) == cudaSuccess) {
+      (e = cudaMalloc(&P->aux_dev, b1 + b2 + b3)) == cudaSuccess) {
     char* d = static_cast<char*>(P->aux_dev);
     std::vector<char> host(b1 + b2);
     std::memcpy(host.data(), P->aux.data(), b1);
@@ -1792,8 +1791,6 @@ int pcg_plan_create(const pcg_hydro_params* prm, int32_t nbox, const pcg_box* bo
     P->d_aux = reinterpret_cast<pcg::AuxBox*>(d);
     P->d_aux_segs = reinterpret_cast<pcg::Seg*>(d + b1);
     P->d_partial = reinterpret_cast<double*>(d + b1 + b2);
-    P->d_done = reinterpret_cast<unsigned*>(d + b1 + b2 + b3);
-    if (e == cudaSuccess) e = cudaMemset(P->d_done, 0, sizeof(unsigned));
   }
   if (e != cudaSuccess) {
     cudaGetLastError();
@@ -1857,9 +1854,6 @@ int pcg_plan_update(pcg_plan* P, const double* dt_dev, pcg_stream_t stream) {
   return e == cudaSuccess ? PCG_OK : fail(PCG_ECUDA, "update: %s", cudaGetErrorString(e));
 }
 
-// Blocks up to which the step tail reduces its own minima: 16 loads per thread of the last one.
-static constexpr int64_t kTailBlocks = 2048;
-
 int pcg_plan_advance(pcg_plan* P, double cfl, const double* dt_dev, double* dt_next, pcg_stream_t stream) {
   if (!P || !dt_dev || !dt_next) return fail(PCG_EINVAL, "bad arguments");
   int rc = ensure_eos(P->prm.nspec);
@@ -1873,20 +1867,12 @@ int pcg_plan_advance(pcg_plan* P, double cfl, const double* dt_dev, double* dt_n
   a.dt_dev = dt_dev;
   a.partial = P->d_partial;
   const int64_t nb = P->L.nblocks[K_CONSUP];
-  // few blocks: the last one takes their minimum itself, which saves a launch; of many, the
-  // cluster of k_estdt_final does it sooner
-  const bool one_launch = nb <= kTailBlocks;
   const bool live = may_overlap(s);
-  a.overlap = overlap_launch(nb, live, live && !one_launch);
-  if (one_launch) {
-    a.done = P->d_done;
-    a.cfl = cfl;
-    a.dt_out = dt_next;
-  }
+  a.overlap = overlap_launch(nb, live, live);
   const int v = variant_of(P->prm.precision_mode, P->prm.nspec, K_CONSUP);
   cudaError_t e = (P->prm.precision_mode == PCG_PREC_FP64) ? pcg_strict::launch_advance(P->prm.nspec, a, nb, v, s)
                                                            : pcg_fast::launch_advance(P->prm.nspec, a, nb, v, s);
-  if (e == cudaSuccess && !one_launch) {
+  if (e == cudaSuccess) {
     pcg::AuxArgs f{};
     f.partial = P->d_partial;
     f.npartial = nb;

@@ -195,11 +195,6 @@ struct StageArgs {
   double difmag;
   const double* dt_dev;  // nullptr: each region's dt
   double* partial;       // fused step tail: one timestep minimum per block
-  // fused step tail of few blocks: the last block to finish (counted in *done, which it
-  // leaves at zero) takes the minimum over all blocks times cfl into *dt_out
-  unsigned* done;        // nullptr: a launch of its own does that
-  double cfl;
-  double* dt_out;
   const void* tmaps;     // TMA-staged trace: 3 tensor maps (x, y, z boxes) per region
   int32_t* err;          // device error word: bit 0 set when a bounded TMA wait gave up
   Seg few[kFewSegs];     // the segments when nseg <= kFewSegs
