@@ -208,9 +208,9 @@ __global__ void __launch_bounds__(128, MINB) k_advance(const __grid_constant__ p
     // itself is never held whole)
     const auto add = [&](int n, double hn) { s[n] = u[n] + dt * hn; };
     if (rg.ff_single)
-      consup_each<NS, float>(rg, it.i, it.j, it.k, p0_of<NS, MIX, float>(rg), add);
+      consup_each<NS, float, true>(rg, it.i, it.j, it.k, p0_of<NS, MIX, float>(rg), add);
     else
-      consup_each<NS, double>(rg, it.i, it.j, it.k, 0.0, add);
+      consup_each<NS, double, false>(rg, it.i, it.j, it.k, 0.0, add);
     dtc = finish_cfl<NS, MIX>(s, rg.dx);
 #pragma unroll
     for (int n = 0; n < pcg::nvar(NS); ++n) u[n] = s[n];

@@ -111,6 +111,16 @@ __device__ __forceinline__ void div_all(const double* x, double b, double* q) {
     div_all<N>(x, b, 1.0 / b, q);
   }
 }
+// One such quotient at a time, r = 1 / b and bok = quot_plain(b) formed once: for a caller
+// that consumes each quotient before it forms the next numerator.
+__device__ __forceinline__ double div_one(double x, double b, double r, bool bok) {
+  if (!(bok && quot_plain(x))) return x / b;
+  const double q0 = x * r;
+  const double q1 = fma(fma(-b, q0, x), r, q0);
+  const double q2 = fma(fma(-b, q1, x), r, q1);
+  const int sign = (__double2hiint(x) ^ __double2hiint(b)) & 0x80000000;
+  return __hiloint2double((__double2hiint(q2) & 0x7fffffff) | sign, __double2loint(q2));
+}
 template <int N>
 __device__ __forceinline__ void div_all(const float* x, float b, float* q) {
 #pragma unroll

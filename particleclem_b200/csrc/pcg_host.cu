@@ -136,7 +136,7 @@ int g_variant[3][3][7] = {
   // one species, 2 to 12 species, more (whose kernels spill under every cap)
   {{0, 0, 2, 0, 2, 1, 2}, {2, 0, 2, 1, 1, 0, 2}, {1, 0, 0, 0, 0, 0, 1}},  // FP64 reference order
   {{0, 0, 2, 0, 0, 0, 0}, {2, 0, 2, 1, 0, 0, 0}, {1, 0, 0, 0, 0, 0, 1}},  // FP64 with FMA
-  {{2, 0, 2, 0, 1, 2, 2}, {2, 0, 0, 0, 1, 2, 2}, {1, 0, 0, 1, 0, 0, 1}},  // mixed
+  {{2, 0, 2, 0, 1, 2, 2}, {2, 0, 0, 0, 1, 1, 2}, {1, 0, 0, 1, 0, 0, 1}},  // mixed
 };
 int species_class(int ns) { return ns == 1 ? 0 : ns <= 12 ? 1 : 2; }
 int max_variant(int prec, int stage) { return (prec == PCG_PREC_MIXED && stage == K_TRACE) ? 5 : 2; }
