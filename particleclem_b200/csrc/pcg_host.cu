@@ -443,10 +443,10 @@ size_t take(Layout& L, const IBox& b, int nc, size_t esz, pcg::View& v, bool blo
 void add_seg(Layout& L, int stage, int region, int variant, const IBox& b) {
   pcg::Seg s{};
   s.region = region;
-  s.variant = variant;
+  s.variant = (int16_t)variant;
   for (int d = 0; d < 3; ++d) { s.lo[d] = b.lo[d]; s.n[d] = (int)b.n(d); }
   s.count = b.cells();
-  s.march = L.march;
+  s.march = (int16_t)L.march;
   s.blk0 = L.nblocks[stage];
   L.segs[stage].push_back(s);
   const bool tiled = stage == K_FLUX2 || (stage == K_FLUX1 && pcg::flux1_shared(L.esz));
@@ -582,13 +582,13 @@ void add_trace_tiles(Layout& L, int region, int d, const IBox& g1) {
   if (!tiles) return;
   pcg::Seg sg{};
   sg.region = region;
-  sg.variant = 3 + d;
+  sg.variant = (int16_t)(3 + d);
   for (int e = 0; e < 3; ++e) {
     sg.lo[e] = g1.lo[e];
     sg.n[e] = (int)(core[e] / tn[e]);
   }
   sg.count = int64_t(sg.n[0]) * sg.n[1] * sg.n[2];
-  sg.march = L.march;
+  sg.march = (int16_t)L.march;
   sg.blk0 = L.nblocks[K_TRACE_TILE];
   L.segs[K_TRACE_TILE].push_back(sg);
   L.nblocks[K_TRACE_TILE] += sg.count;
@@ -597,17 +597,15 @@ void add_trace_tiles(Layout& L, int region, int d, const IBox& g1) {
 // Faces each thread of a marching stage takes in turn along y or z. A march shares the
 // correction of the cell between two faces (4 faces need 5 corrections, 4 single faces 8),
 // but its faces come one after the other, and a small call leaves the chip idle meanwhile:
-// then shorter marches on more threads finish sooner.
-#ifndef PCG_MARCH_CELLS1
-#define PCG_MARCH_CELLS1 60000
-#endif
-#ifndef PCG_MARCH_CELLS2
-#define PCG_MARCH_CELLS2 120000
-#endif
+// then shorter marches on more threads finish sooner. Replayed steps of one-box levels, marches
+// of 1 / 2 / 4 faces, us: one species mixed 32^3 55.9 / 61.5 / 75.1, 40^3 72.5 / 71.8 / 86.0,
+// 48^3 102 / 99.5 / 107, 56^3 147 / 141 / 139; 9 species FP64 36^3 270 / 260 / 286, 40^3 320 /
+// 319 / 334, 48^3 520 / 505 / 515, 64^3 958 / 941 / 942.
+constexpr int64_t kMarchCells1 = 60000, kMarchCells2 = 120000;
 int face_march(const std::vector<BoxIn>& boxes) {
   int64_t cells = 0;
   for (const BoxIn& b : boxes) cells += b.bx.cells();
-  return cells <= PCG_MARCH_CELLS1 ? 1 : cells <= PCG_MARCH_CELLS2 ? 2 : pcg::FACE_MARCH;
+  return cells <= kMarchCells1 ? 1 : cells <= kMarchCells2 ? 2 : pcg::FACE_MARCH;
 }
 
 void build_layout(Layout& L, const std::vector<BoxIn>& boxes, const pcg_hydro_params* prm) {
@@ -830,34 +828,37 @@ bool encode_trace_maps(const pcg::Region& R, int nc, char* out) {
   return true;
 }
 
-// encode = false: sizing only, before the workspace addresses exist (no tensor maps).
-void pack_tables(const Layout& L, Tables& T, bool encode = true) {
+// Offsets of a call's tables within one block, its size in T.bytes.
+void size_tables(const Layout& L, Tables& T) {
   static_assert(sizeof(CUtensorMap) == pcg::kTensorMapBytes, "CUtensorMap size");
   size_t off = L.regions.size() * sizeof(pcg::Region);
-  size_t seg_off[K_NKIND];
   for (int s = 0; s < K_NKIND; ++s) {
     off = (off + 15) / 16 * 16;
-    seg_off[s] = off;
+    T.segs[s] = reinterpret_cast<const pcg::Seg*>(off);
     off += L.segs[s].size() * sizeof(pcg::Seg);
   }
   off = (off + 127) / 128 * 128;  // tensor maps: 64-byte aligned (the table base is 256-aligned)
-  const size_t map_off = off;
+  T.tmaps = reinterpret_cast<const void*>(off);
   if (L.tile_trace) off += L.regions.size() * 3 * pcg::kTensorMapBytes;
-  const size_t err_off = off;
-  off += 16;
-  T.bytes = off;
+  T.err = reinterpret_cast<int32_t*>(off);
+  T.bytes = off + 16;
+}
+
+// The tables' host copy, once the regions hold their workspace addresses.
+void pack_tables(const Layout& L, Tables& T) {
+  size_tables(L, T);
   T.host.assign(T.bytes, 0);
   if (!L.regions.empty()) std::memcpy(T.host.data(), L.regions.data(), L.regions.size() * sizeof(pcg::Region));
   for (int s = 0; s < K_NKIND; ++s)
-    if (!L.segs[s].empty()) std::memcpy(T.host.data() + seg_off[s], L.segs[s].data(), L.segs[s].size() * sizeof(pcg::Seg));
-  T.maps_ok = L.tile_trace && encode;
+    if (!L.segs[s].empty())
+      std::memcpy(T.host.data() + reinterpret_cast<size_t>(T.segs[s]), L.segs[s].data(),
+                  L.segs[s].size() * sizeof(pcg::Seg));
+  const size_t map_off = reinterpret_cast<size_t>(T.tmaps);
+  T.maps_ok = L.tile_trace;
   for (size_t r = 0; r < L.regions.size() && T.maps_ok; ++r)
     T.maps_ok = encode_trace_maps(L.regions[r], pcg::nt_comps(L.ns),
                                   T.host.data() + map_off + r * 3 * pcg::kTensorMapBytes);
-  // device pointers are filled in by bind_tables once T.dev exists
-  for (int s = 0; s < K_NKIND; ++s) T.segs[s] = reinterpret_cast<const pcg::Seg*>(seg_off[s]);
-  T.tmaps = reinterpret_cast<const void*>(map_off);
-  T.err = reinterpret_cast<int32_t*>(err_off);
+  // the offsets become device pointers in bind_tables, once T.dev exists
 }
 
 void bind_tables(Tables& T) {
@@ -947,33 +948,31 @@ int launch_stages(const Layout& L, const Tables& T, const pcg_hydro_params* p, i
   return PCG_OK;
 }
 
-// One-shot execution: stream-ordered workspace and tables, launches, stream-ordered free.
+// One-shot execution: stream-ordered workspace and tables (one allocation: two of each call
+// cost a small one-shot call a few microseconds of host time), launches, stream-ordered free.
 int run_once(const pcg_hydro_params* p, std::vector<BoxIn>& boxes, int first, int last, cudaStream_t s) {
   int rc = ensure_eos(p->nspec);
   if (rc) return rc;
   Layout L;
   build_layout(L, boxes, p);
   if (L.oversize) return fail(PCG_EINVAL, "a region needs workspace arrays of 2^31 elements or more: use smaller boxes");
-  void* ws = nullptr;
-  if (L.ws_bytes) CUDA_TRY(ws_alloc(&ws, L.ws_bytes, s));
-  rebase_workspace(L, boxes, static_cast<char*>(ws));
+  // one stream-ordered allocation: [workspace | tables]
   Tables T;
+  size_tables(L, T);
+  const size_t off_t = (L.ws_bytes + kAlign - 1) / kAlign * kAlign;
+  void* mem = nullptr;
+  CUDA_TRY(ws_alloc(&mem, off_t + T.bytes, s));
+  rebase_workspace(L, boxes, static_cast<char*>(mem));
   pack_tables(L, T);
-  cudaError_t e = ws_alloc(&T.dev, T.bytes, s);
-  if (e != cudaSuccess) {
-    if (ws) cudaFreeAsync(ws, s);
-    cudaGetLastError();
-    return fail(PCG_ENOMEM, "table allocation: %s", cudaGetErrorString(e));
-  }
-  e = upload(T.dev, T.host.data(), T.bytes, s);
+  T.dev = static_cast<char*>(mem) + off_t;
+  cudaError_t e = upload(T.dev, T.host.data(), T.bytes, s);
   if (e == cudaSuccess) {
     bind_tables(T);
     rc = launch_stages(L, T, p, first, last, nullptr, s);
   } else {
     rc = fail(PCG_ECUDA, "table upload: %s", cudaGetErrorString(e));
   }
-  cudaFreeAsync(T.dev, s);
-  if (ws) cudaFreeAsync(ws, s);
+  cudaFreeAsync(mem, s);
   return rc;
 }
 
@@ -1470,7 +1469,7 @@ int pcg_step_boxes(const pcg_hydro_params* prm, int32_t nbox, const pcg_box* box
   }
   // one stream-ordered allocation: [workspace | tables | fill table | block minima]
   Tables T;
-  pack_tables(L, T, false);
+  size_tables(L, T);
   const size_t off_t = (L.ws_bytes + kAlign - 1) / kAlign * kAlign;
   const size_t off_f = off_t + (T.bytes + kAlign - 1) / kAlign * kAlign;
   const size_t off_p = off_f + (fills.size() * sizeof(pcg::FillBox) + kAlign - 1) / kAlign * kAlign;
@@ -1546,7 +1545,7 @@ int pcg_hydro_workspace(const pcg_hydro_params* prm, int32_t nbox, const int32_t
   build_layout(L, bs, prm);
   if (L.oversize) return fail(PCG_EINVAL, "a region needs workspace arrays of 2^31 elements or more: use smaller boxes");
   Tables T;
-  pack_tables(L, T, false);
+  size_tables(L, T);
   *bytes = int64_t(size_class((L.ws_bytes + kAlign - 1) / kAlign * kAlign + T.bytes));  // as ws_alloc takes it
   return PCG_OK;
 }
@@ -2042,7 +2041,7 @@ extern "C" int pcg_hydro_box_noalloc(const pcg_hydro_params* prm, const int32_t 
   if (L.oversize) return fail(PCG_EINVAL, "box too large");
   // scratch = [tables | workspace]; the table size does not depend on the addresses
   Tables T;
-  pack_tables(L, T, false);
+  size_tables(L, T);
   const size_t ws_off = (T.bytes + kAlign - 1) / kAlign * kAlign;
   const size_t need = ws_off + L.ws_bytes;
   if (need > kNoAllocScratchBytes)

@@ -165,11 +165,10 @@ PCG_HD constexpr bool flux1_shared(size_t esz) { return esz == 4; }
 
 struct Seg {
   int32_t region;
-  int32_t variant;
+  int16_t variant;
+  int16_t march;  // faces per thread along y and z in the stages that march
   int32_t lo[3];
   int32_t n[3];
-  int32_t march;  // faces per thread along y and z in the stages that march
-  int32_t pad;
   int64_t count;
   int64_t blk0;  // first block of this segment within the launch
 };

@@ -5,8 +5,8 @@ it reads and every output element it writes, each counted once per launch (no st
 re-reads). For a region of valid edges (nx, ny, nz), NS species, compute-type size
 ``r`` (8 FP64, 4 mixed) and NT = 6 + NS, NF = 7 + NS, NVAR = 7 + NS, QVAR = 8 + NS:
 
-* ctoprim: read NVAR doubles and write QVAR + 6 doubles per cell of grow(box, 4); the
-           mixed form (r = 4) also writes the FP32 copy of NT primitives on grow(box, 3)
+* ctoprim: read NVAR doubles and write 2 auxiliary doubles (gamma_c, c) and the primitives
+           per cell of grow(box, 4): QVAR - 2 doubles, or NT floats in the mixed form (r = 4)
 * prep:    read (5 + NS) q doubles per cell of grow(box, 4); write 2 r per cell of
            grow(box, 1) and one double per node of the box
 * trace:   read (5 + NS) q doubles per cell of grow(box, 3) (PLM: 6 + NS); write
@@ -30,7 +30,7 @@ import json
 import os
 import re
 
-FALLBACK_HBM_GBS = 6650.0  # earlier measurement on this pool, used only without MEASURED_PEAKS.json
+FALLBACK_HBM_GBS = 6650.0  # an earlier copy measurement, used only without a measured peaks file
 
 
 def peaks(root):
@@ -57,7 +57,8 @@ def stage_bytes(stage, n, ns, r, ppm=True):
     nt, nf, nv, nq = 6 + ns, 7 + ns, 7 + ns, 8 + ns
     ff = 4 if r == 4 else 8  # final-flux element size
     if stage == "ctoprim":
-        return _cells(n, 4) * 8 * (nv + nq + 6) + (_cells(n, 3) * nt * 4 if r == 4 else 0)
+        # the stages' own copies: no T, GAME in q; gamma_c and c of the auxiliary state
+        return _cells(n, 4) * (8 * (nv + 2) + (nt * 4 if r == 4 else 8 * (nq - 2)))
     if stage == "prep":
         nodes = (n[0] + 1) * (n[1] + 1) * (n[2] + 1)
         return _cells(n, 4) * 8 * (5 + ns) + _cells(n, 1) * 2 * r + nodes * 8
