@@ -340,7 +340,7 @@ int pcg_average_down(const pcg_array4* fine, pcg_array4* crse, const int32_t fin
 
 /* Each heavy stage (0 ctoprim, 2 trace, 3-5 Riemann stages) exists in three register
  * budgets (variants 0-2, increasingly tight); the library keeps the variant used
- * per (precision_mode, species class of nspec: 1, 2-12 or more, stage). The trace of
+ * per (precision_mode, species class of nspec: 1, 2-5, 6-12 or more, stage). The trace of
  * PCG_PREC_MIXED has variants 3-5 as well: the same budgets for the tiled trace, which stages each tile of the FP32
  * primitive state and its halo in shared memory with one TMA load (plain PPM and PLM;
  * the hybrid-WENO trace is never tiled). particleclem_b200/autotune.py times them and

@@ -132,17 +132,33 @@ thread_local std::string g_err;
 // register budgets 0-2.
 constexpr int kTileVariant = 3;
 std::mutex g_var_mu;
-int g_variant[3][3][7] = {
-  // one species, 2 to 12 species, more (whose kernels spill under every cap)
-  {{0, 0, 2, 0, 2, 1, 2}, {2, 0, 2, 1, 1, 0, 2}, {1, 0, 0, 0, 0, 0, 1}},  // FP64 reference order
-  {{0, 0, 2, 0, 0, 0, 0}, {2, 0, 2, 1, 0, 0, 0}, {1, 0, 0, 0, 0, 0, 1}},  // FP64 with FMA
-  {{2, 0, 2, 0, 1, 2, 2}, {2, 0, 0, 0, 1, 1, 2}, {1, 0, 0, 1, 0, 0, 1}},  // mixed
+int g_variant[3][4][7] = {
+  // one species, 2 to 5 species, 6 to 12, more (whose kernels spill under every cap)
+  {{0, 0, 2, 0, 2, 1, 2}, {2, 0, 1, 2, 2, 2, 1}, {2, 0, 2, 1, 0, 0, 2}, {1, 0, 0, 0, 0, 0, 1}},  // FP64 reference order
+  {{0, 0, 2, 0, 0, 0, 0}, {2, 0, 1, 2, 2, 2, 1}, {2, 0, 2, 1, 0, 0, 0}, {1, 0, 0, 0, 0, 0, 1}},  // FP64 with FMA
+  {{2, 0, 2, 0, 1, 2, 2}, {2, 0, 0, 0, 2, 2, 1}, {2, 0, 0, 0, 1, 1, 2}, {1, 0, 0, 1, 0, 0, 1}},  // mixed
 };
-int species_class(int ns) { return ns == 1 ? 0 : ns <= 12 ? 1 : 2; }
+// Mixtures of few species hold their states in fewer registers, so the tighter caps of the set
+// pay: 104^3, 3 species, ms per launch at the caps of 9 species -> at theirs: FP64 flux2 0.550 ->
+// 0.461, with FMA flux1 0.528 -> 0.447, flux2 0.458 -> 0.396, mixed flux1 0.278 -> 0.214. Counts
+// measured: 2 and 3 alike, 9, 21. A launch of one wave (4 blocks per SM, in the FP64 forms, whose
+// tight caps spill more, two such waves) has little to gain from them and takes the next class's
+// caps unless the caller chose the variant. Steps of 3-species levels, us, next class -> tight: 16^3
+// FP64 81.2 -> 83.5, mixed 64.0 -> 64.2; 30^3 FP64 112 -> 120; 34^3 137 -> 143; 36^3 147 -> 144;
+// 48^3 286 -> 260; 33^3 mixed (hybrid WENO) 94.0 -> 86.8.
+enum { FEW_SPECIES = 1 };
+constexpr int kFewBlocksVariant[3][7] = {{2, 0, 2, 1, 1, 0, 2}, {2, 0, 2, 1, 0, 0, 0}, {2, 0, 0, 0, 1, 1, 2}};
+constexpr int64_t kFewBlocks[3] = {8 * 148, 8 * 148, 4 * 148};
+bool g_chosen[3][4][7];
+int species_class(int ns) { return ns == 1 ? 0 : ns <= 5 ? FEW_SPECIES : ns <= 12 ? 2 : 3; }
 int max_variant(int prec, int stage) { return (prec == PCG_PREC_MIXED && stage == K_TRACE) ? 5 : 2; }
-int variant_of(int prec, int ns, int stage) {
+// The variant of a launch of nblocks blocks.
+int variant_of(int prec, int ns, int stage, int64_t nblocks) {
   std::lock_guard<std::mutex> lk(g_var_mu);
-  return g_variant[prec][species_class(ns)][stage];
+  const int cls = species_class(ns);
+  if (cls == FEW_SPECIES && nblocks <= kFewBlocks[prec] && !g_chosen[prec][cls][stage])
+    return kFewBlocksVariant[prec][stage];
+  return g_variant[prec][cls][stage];
 }
 
 // Stream-ordered workspace pool per device. Its release threshold is unbounded, so
@@ -926,7 +942,7 @@ int launch_segs(const Layout& L, const Tables& T, const pcg_hydro_params* p, int
 
 int launch_kind(const Layout& L, const Tables& T, const pcg_hydro_params* p, int kind, const double* dt_dev,
                 bool after, bool more, cudaStream_t s) {
-  int var = kind < K_NSTAGE ? variant_of(p->precision_mode, L.ns, kind) : 0;
+  int var = kind < K_NSTAGE ? variant_of(p->precision_mode, L.ns, kind, L.nblocks[kind]) : 0;
   if (var >= kTileVariant) {
     var -= kTileVariant;
     // the mixed form's tiled trace (variants 3-5), when every tensor map was encoded
@@ -1511,7 +1527,7 @@ int pcg_step_boxes(const pcg_hydro_params* prm, int32_t nbox, const pcg_box* box
     set_segs(a, L.segs[K_CONSUP]);
     a.partial = partial;
     a.overlap = overlap_launch(L.nblocks[K_CONSUP], live, live);
-    const int v = variant_of(prm->precision_mode, prm->nspec, K_CONSUP);
+    const int v = variant_of(prm->precision_mode, prm->nspec, K_CONSUP, L.nblocks[K_CONSUP]);
     e = strict ? pcg_strict::launch_advance(prm->nspec, a, L.nblocks[K_CONSUP], v, s)
                : pcg_fast::launch_advance(prm->nspec, a, L.nblocks[K_CONSUP], v, s);
     if (e == cudaSuccess) {
@@ -1868,7 +1884,7 @@ int pcg_plan_advance(pcg_plan* P, double cfl, const double* dt_dev, double* dt_n
   const int64_t nb = P->L.nblocks[K_CONSUP];
   const bool live = may_overlap(s);
   a.overlap = overlap_launch(nb, live, live);
-  const int v = variant_of(P->prm.precision_mode, P->prm.nspec, K_CONSUP);
+  const int v = variant_of(P->prm.precision_mode, P->prm.nspec, K_CONSUP, nb);
   cudaError_t e = (P->prm.precision_mode == PCG_PREC_FP64) ? pcg_strict::launch_advance(P->prm.nspec, a, nb, v, s)
                                                            : pcg_fast::launch_advance(P->prm.nspec, a, nb, v, s);
   if (e == cudaSuccess) {
@@ -1935,13 +1951,14 @@ int pcg_set_launch_variant(int32_t precision_mode, int32_t nspec, int32_t stage,
     return fail(PCG_EINVAL, "launch variant (%d, %d, %d, %d) out of range", precision_mode, nspec, stage, variant);
   std::lock_guard<std::mutex> lk(g_var_mu);
   g_variant[precision_mode][species_class(nspec)][stage] = variant;
+  g_chosen[precision_mode][species_class(nspec)][stage] = true;
   return PCG_OK;
 }
 
 int pcg_get_launch_variant(int32_t precision_mode, int32_t nspec, int32_t stage) {
   if (precision_mode < 0 || precision_mode > 2 || !species_built(nspec) || stage < 0 || stage >= K_NSTAGE)
     return fail(PCG_EINVAL, "launch variant query out of range");
-  return variant_of(precision_mode, nspec, stage);
+  return variant_of(precision_mode, nspec, stage, INT64_MAX);
 }
 
 int pcg_plan_destroy(pcg_plan* P) {
