@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from common import MIXED_TOL, eos9, gpu_zeros, oracle, params_for, rel_err, to_cpu, to_gpu
-from particleclem_b200 import abi, hydro, workloads as wl
+from particleclem_b200 import abi, hydro, thermo, workloads as wl
 
 pytestmark = pytest.mark.gpu
 FORMS = [abi.PREC_FP64, abi.PREC_FP64_FAST, abi.PREC_MIXED]
@@ -155,3 +155,22 @@ def test_timestep_reduction_equals_the_oracle(edges):
     dt = torch.zeros(1, dtype=torch.float64, device="cuda")
     hydro.estdt(1, [hydro.make_box(p.lo, p.hi, to_gpu(p.fab), None, p.dx, 0.0)], 0.4, dt)
     assert dt.item() == 0.4 * oracle().estdt(p.lo, p.hi, p.fab, p.dx)
+
+
+@pytest.mark.parametrize("nspec", [2, 3])
+@pytest.mark.parametrize("edges", [(35, 34, 33), (44, 41, 39)])
+def test_few_species_equal_oracle_on_both_sides_of_the_launch_size_rule(nspec, edges):
+    """Launches of up to 1184 blocks (128 faces each) and larger ones run the FP64
+    stages of 2 to 5 species at different register caps."""
+    if nspec not in hydro.species_counts():
+        pytest.skip(f"library built without {nspec} species")
+    eos = thermo.standin_mixture(nspec)
+    hydro.init(0)
+    hydro.set_eos(eos)
+    oracle().set_eos(eos)
+    p = wl.random_patch(edges, 17, eos)
+    prm = params_for(p, 0.3 * oracle().estdt(p.lo, p.hi, p.fab, p.dx), prec=abi.PREC_FP64, nspec=nspec)
+    ref, _ = oracle().hydro_box(prm, p.lo, p.hi, p.fab)
+    out = gpu_zeros(abi.nvar(nspec), p.lo, p.hi)
+    hydro.hydro_box(prm, p.lo, p.hi, to_gpu(p.fab), out)
+    np.testing.assert_array_equal(to_cpu(out), ref.data)
