@@ -190,10 +190,11 @@ __global__ void __launch_bounds__(128) k_update(const __grid_constant__ pcg::Aux
 }
 
 // The tail of a level step in one pass over the cells of each region: the flux
-// divergence and p div u of pc_consup (kept in registers, the hydro source array is not
+// divergence of pc_consup (kept in registers, the hydro source array is not
 // written), S_new = S_old + dt * hydro_source with computeTemp written over the state in
 // place, and the CFL constraint of S_new for the next step (block minima; the final
-// minimum is k_estdt_final). Each value is formed by the same expressions as k_consup,
+// minimum is k_estdt_final). In place: a thread reads and writes the state of its own cell
+// only. Each value is formed by the same expressions as k_consup,
 // k_update and k_estdt, so the step is the unfused step's.
 template <int NS, bool MIX, int MINB>
 __global__ void __launch_bounds__(128, MINB) k_advance(const __grid_constant__ pcg::StageArgs a) {
@@ -205,12 +206,14 @@ __global__ void __launch_bounds__(128, MINB) k_advance(const __grid_constant__ p
     const CellPtr<double> u = at(v4<double>(rg.uin), it.i, it.j, it.k);
     const double dt = dt_of(a, rg);
     // S_old + dt * hydro source, each component as its source is formed (the source
-    // itself is never held whole)
+    // itself is never held whole). UEINT is left out: finish_cfl forms it from the total
+    // energy. The p div u term it would carry adds the region's pressure offset (p0_of), a read of
+    // another cell of the state this launch is replacing.
     const auto add = [&](int n, double hn) { s[n] = u[n] + dt * hn; };
     if (rg.ff_single)
-      consup_each<NS, float, true>(rg, it.i, it.j, it.k, p0_of<NS, MIX, float>(rg), add);
+      consup_each<NS, float, true, false>(rg, it.i, it.j, it.k, 0.0, add);
     else
-      consup_each<NS, double, false>(rg, it.i, it.j, it.k, 0.0, add);
+      consup_each<NS, double, false, false>(rg, it.i, it.j, it.k, 0.0, add);
     dtc = finish_cfl<NS, MIX>(s, rg.dx);
 #pragma unroll
     for (int n = 0; n < pcg::nvar(NS); ++n) u[n] = s[n];

@@ -1854,29 +1854,31 @@ template <int NC> struct FinalView<float, NC> {
 // The hydro source of cell (i, j, k), component by component: out(n, h_n) for n = 0 ..
 // NVAR-1 (the p div u term already in h_UEINT), so that a caller can consume each
 // component as it is formed instead of holding all of them. TOGETHER: the flux sums are
-// formed first and divided by the volume together, else component by component.
-template <int NS, class F, bool TOGETHER, class OUT>
+// formed first and divided by the volume together, else component by component. EINT false
+// leaves UEINT out, and with it the p div u term, the face states and p0: the step tail
+// replaces that component by the total energy's.
+template <int NS, class F, bool TOGETHER, bool EINT, class OUT>
 __device__ __forceinline__ void consup_each(const pcg::Region& rg, int i, int j, int k, double p0, OUT&& out) {
   constexpr int NV = pcg::nvar(NS);
   const FinalView<F, NV> f0(rg.ff[0], 0, i, j, k), f1(rg.ff[1], 1, i, j, k), f2(rg.ff[2], 2, i, j, k);
-  const FinalView<F, 2> e0(rg.qec[0], 0, i, j, k), e1(rg.qec[1], 1, i, j, k), e2(rg.qec[2], 2, i, j, k);
-  constexpr int VE = FinalView<F, 2>::V;
-  double q0[2], q0p[2], q1[2], q1p[2], q2[2], q2p[2];
-#pragma unroll
-  for (int n0 = 0; n0 < 2; n0 += VE) {
-    e0.get(n0, q0 + n0, q0p + n0);
-    e1.get(n0, q1 + n0, q1p + n0);
-    e2.get(n0, q2 + n0, q2p + n0);
-  }
-  const bool ua = rg.area[0].p != nullptr;
-  const V4<const double> a0 = v4<const double>(rg.area[0]);
-  const V4<const double> a1 = v4<const double>(rg.area[1]);
-  const V4<const double> a2 = v4<const double>(rg.area[2]);
-  const double a0m = ua ? a0(i, j, k) : rg.area_u[0], a0p = ua ? a0(i + 1, j, k) : rg.area_u[0];
-  const double a1m = ua ? a1(i, j, k) : rg.area_u[1], a1p = ua ? a1(i, j + 1, k) : rg.area_u[1];
-  const double a2m = ua ? a2(i, j, k) : rg.area_u[2], a2p = ua ? a2(i, j, k + 1) : rg.area_u[2];
   const double v = rg.vol.p ? v4<const double>(rg.vol)(i, j, k) : rg.vol_u;
   const auto pdivu_sum = [&] {
+    const FinalView<F, 2> e0(rg.qec[0], 0, i, j, k), e1(rg.qec[1], 1, i, j, k), e2(rg.qec[2], 2, i, j, k);
+    constexpr int VE = FinalView<F, 2>::V;
+    double q0[2], q0p[2], q1[2], q1p[2], q2[2], q2p[2];
+#pragma unroll
+    for (int n0 = 0; n0 < 2; n0 += VE) {
+      e0.get(n0, q0 + n0, q0p + n0);
+      e1.get(n0, q1 + n0, q1p + n0);
+      e2.get(n0, q2 + n0, q2p + n0);
+    }
+    const bool ua = rg.area[0].p != nullptr;
+    const V4<const double> a0 = v4<const double>(rg.area[0]);
+    const V4<const double> a1 = v4<const double>(rg.area[1]);
+    const V4<const double> a2 = v4<const double>(rg.area[2]);
+    const double a0m = ua ? a0(i, j, k) : rg.area_u[0], a0p = ua ? a0(i + 1, j, k) : rg.area_u[0];
+    const double a1m = ua ? a1(i, j, k) : rg.area_u[1], a1p = ua ? a1(i, j + 1, k) : rg.area_u[1];
+    const double a2m = ua ? a2(i, j, k) : rg.area_u[2], a2p = ua ? a2(i, j, k + 1) : rg.area_u[2];
     return 0.5 * ((q0p[0] + p0 + (q0[0] + p0)) * (q0p[1] * a0p - q0[1] * a0m) +
                   (q1p[0] + p0 + (q1[0] + p0)) * (q1p[1] * a1p - q1[1] * a1m) +
                   (q2p[0] + p0 + (q2[0] + p0)) * (q2p[1] * a2p - q2[1] * a2m));
@@ -1887,7 +1889,10 @@ __device__ __forceinline__ void consup_each(const pcg::Region& rg, int i, int j,
   // tail 0.273 together, 0.212 one by one; its FP32 fluxes come in groups, together).
   constexpr int V = FinalView<F, NV>::V;
   if constexpr (TOGETHER || V > 1) {
-    double num[NV + 1];
+    // the numerators in component order, p div u last; without EINT neither it nor UEINT
+    constexpr int NUM = EINT ? NV + 1 : NV - 1;
+    const auto slot = [](int n) { return EINT || n < pcg::UEINT ? n : n - 1; };
+    double num[NUM];
 #pragma unroll
     for (int n0 = 0; n0 < NV; n0 += V) {
       double xm[V], xp[V], ym[V], yp[V], zm[V], zp[V];
@@ -1896,25 +1901,29 @@ __device__ __forceinline__ void consup_each(const pcg::Region& rg, int i, int j,
       f2.get(n0, zm, zp);
 #pragma unroll
       for (int m = 0; m < V; ++m)
-        if (n0 + m < NV) num[n0 + m] = xm[m] - xp[m] + ym[m] - yp[m] + zm[m] - zp[m];
+        if (n0 + m < NV && (EINT || n0 + m != pcg::UEINT))
+          num[slot(n0 + m)] = xm[m] - xp[m] + ym[m] - yp[m] + zm[m] - zp[m];
     }
-    num[NV] = pdivu_sum();
-    div_all<NV + 1>(num, v, num);
+    if constexpr (EINT) num[NV] = pdivu_sum();
+    div_all<NUM>(num, v, num);
     const CellPtr<double> uo = at(v4<double>(rg.uout), i, j, k);
 #pragma unroll
     for (int n = 0; n < NV; ++n) {
+      if (!EINT && n == pcg::UEINT) continue;
       const double old = rg.zero_uout ? 0.0 : uo[n];
-      double h = old + num[n];
-      if (n == pcg::UEINT) h -= num[NV];
+      double h = old + num[slot(n)];
+      if (n == pcg::UEINT) h -= num[NUM - 1];
       out(n, h);
     }
   } else {
     const double r = 1.0 / v;
     const bool vok = quot_plain(v) && v != 0.0;
-    const double pdivu = div_one(pdivu_sum(), v, r, vok);
+    double pdivu = 0.0;
+    if constexpr (EINT) pdivu = div_one(pdivu_sum(), v, r, vok);
     const CellPtr<double> uo = at(v4<double>(rg.uout), i, j, k);
 #pragma unroll
     for (int n = 0; n < NV; ++n) {
+      if (!EINT && n == pcg::UEINT) continue;
       double xm, xp, ym, yp, zm, zp;
       f0.get(n, &xm, &xp);
       f1.get(n, &ym, &yp);
@@ -1929,7 +1938,7 @@ __device__ __forceinline__ void consup_each(const pcg::Region& rg, int i, int j,
 
 template <int NS, class F>
 __device__ __forceinline__ void consup_sum(const pcg::Region& rg, int i, int j, int k, double p0, double* h) {
-  consup_each<NS, F, true>(rg, i, j, k, p0, [&](int n, double hn) { h[n] = hn; });
+  consup_each<NS, F, true, true>(rg, i, j, k, p0, [&](int n, double hn) { h[n] = hn; });
 }
 
 template <int NS, class F>
