@@ -472,16 +472,18 @@ void add_seg(Layout& L, int stage, int region, int variant, const IBox& b) {
 // Work order within a launch. Blocks start roughly in launch order, so the order of the
 // segments decides which data is live in L2 at the same time.
 // (1) The final fluxes of all three directions read the state and the nodal div u
-// (artificial viscosity). In a region whose state would not stay in L2 between its
-// direction segments (kOrderRegionBytes) the k_flux2 direction segments are therefore
-// interleaved in slabs of kOrderSlab z-planes (x, y, z of one slab, then the next slab)
-// so that a slab's state comes from DRAM once. Measured on the 128^3 flame level (mixed
-// form): flux2 0.672 -> 0.657 ms, later 0.628 -> 0.616. With one species the state is a smaller
-// part of what flux2 reads and the three directions' code competes for the instruction caches
-// (256^3, mixed: 2.35 -> 2.49 ms), so one-species regions keep whole directions. The same interleave slowed the stages whose
-// directions run different code (flux1 0.661 -> 0.726 ms, trace 0.631 -> 0.658, flux0
-// 0.228 -> 0.245), so they keep one segment per direction (PCG_ORDER_SLABS: bit K_* of
-// the stages that interleave).
+// (artificial viscosity). In the mixed form of a mixture, the k_flux2 direction segments of a
+// region whose state would not stay in L2 between them (kOrderRegionBytes) are therefore
+// interleaved in slabs of kOrderSlab z-planes (x, y, z of one slab, then the next slab), so
+// that a slab's state comes from DRAM once. ms, whole directions / slabs: one box of 96^3, 9
+// species 0.305 / 0.287, 128^3 0.670 / 0.650, four boxes of 96^3 1.150 / 1.087, 128^3 with 3
+// species 0.459 / 0.436. The FP64 kernels' directions are more code and lose more to the
+// instruction caches than the state's second read costs (9 species, 128^3: 1.702 / 2.067,
+// 96^3 0.743 / 0.809, with FMA 1.364 / 1.605; 21 species, 80^3: 1.49 / 2.33), and with one
+// species the state is a smaller part of what flux2 reads (256^3, mixed: 2.35 / 2.49), so these
+// keep whole directions. The same interleave slowed the mixed stages whose directions run
+// different code (flux1 0.661 / 0.726, trace 0.631 / 0.658, flux0 0.228 / 0.245), so they keep
+// one segment per direction (PCG_ORDER_SLABS: bit K_* of the stages that interleave).
 // (2) Successive stages alternate their traversal direction (prep, flux0 and flux2 run
 // their segments in reverse order, PCG_ORDER_REVERSE), so that the data a stage wrote
 // last, still in L2, is what the next stage reads first (step 2.960 -> 2.953 ms alone,
@@ -558,9 +560,8 @@ void reverse_segs(Layout& L, int stage) {
 
 // Order the segments of a stage by direction (x of every region, then y, then z), block
 // offsets renumbered. Each direction is its own code, and with a few blocks of every region
-// resident all three compete for an SM's instruction caches. 64 boxes of 32^3, 9 species, FP64:
-// flux0 0.795 -> 0.717 ms, flux1 2.25 -> 2.07, flux2 1.72 -> 1.48; the trace, whose directions
-// share the primitives they read, 1.478 -> 1.504, so it keeps its order.
+// resident all three compete for an SM's instruction caches; in region order, a region's
+// directions find what they share in L2. group_by_direction picks.
 void group_segs(Layout& L, int stage) {
   std::vector<pcg::Seg>& v = L.segs[stage];
   const size_t n = v.size();
@@ -573,6 +574,34 @@ void group_segs(Layout& L, int stage) {
     v[i].blk0 = b;
     b += w[i].second;
   }
+}
+
+// Which of the two orders a call of many regions takes, by the size of its regions (mean
+// cells). The large kernels (FP64 in reference order, and with FMA from 6 species) always gain
+// from whole directions; the smaller ones only while a region's direction is too few blocks
+// to fill the chip, flux1 up to larger regions than flux0 and flux2; with one species only in
+// calls of a few waves. ms, region order / by direction, flux0, flux1, flux2:
+//   9 species FP64   64 x 32^3  1.03 / .940   3.21 / 2.91   2.03 / 1.92
+//                     8 x 64^3  .978 / .854   2.73 / 2.68   1.99 / 1.84
+//   9 species mixed 300 x 12^3  .146 / .130   .403 / .334   .283 / .256
+//                    40 x 24^3  .113 / .107   .297 / .274   .229 / .227
+//                    40 x 28^3  .158 / .156   .440 / .404   .336 / .342
+//                    64 x 32^3  .344 / .347   .933 / .881   .702 / .762
+//                     6 x 56^3  .143 / .157   .418 / .420   .342 / .363
+//   3 species mixed  24 x 32^3  .090 / .088   .223 / .207   .197 / .203
+//                     6 x 64^3  .133 / .137   .339 / .342   .334 / .360
+//   2 species FMA    16 x 40^3  .151 / .150   .436 / .410   .344 / .356
+//   one species FP64 32 x 16^3  .027 / .027   .060 / .057   .061 / .051
+//                    64 x 32^3  .253 / .264   .632 / .650   .576 / .611
+//   one species mixed 8 x 32^3  .023 / .023   .057 / .053   .055 / .051
+//                    64 x 32^3  .143 / .150   .352 / .378   .329 / .375
+constexpr int64_t kGroupCells = 20000, kGroupCellsFlux1 = 200000;
+constexpr int64_t kGroupCellsOne = 40000, kGroupCallCellsOne = int64_t(1) << 18;
+bool group_by_direction(int prec, int ns, int stage, int64_t regions, int64_t cells) {
+  if (regions < 2) return false;
+  if (ns == 1) return cells / regions <= kGroupCellsOne && cells <= kGroupCallCellsOne;
+  if (prec == PCG_PREC_FP64 || (prec == PCG_PREC_FP64_FAST && ns > 5)) return true;
+  return cells / regions <= (stage == K_FLUX1 ? kGroupCellsFlux1 : kGroupCells);
 }
 
 // The tiled trace of direction d over g1 = grow(box,1), as K_TRACE_TILE segments: the up
@@ -618,9 +647,7 @@ void add_trace_tiles(Layout& L, int region, int d, const IBox& g1) {
 // 48^3 102 / 99.5 / 107, 56^3 147 / 141 / 139; 9 species FP64 36^3 270 / 260 / 286, 40^3 320 /
 // 319 / 334, 48^3 520 / 505 / 515, 64^3 958 / 941 / 942.
 constexpr int64_t kMarchCells1 = 60000, kMarchCells2 = 120000;
-int face_march(const std::vector<BoxIn>& boxes) {
-  int64_t cells = 0;
-  for (const BoxIn& b : boxes) cells += b.bx.cells();
+int face_march(int64_t cells) {
   return cells <= kMarchCells1 ? 1 : cells <= kMarchCells2 ? 2 : pcg::FACE_MARCH;
 }
 
@@ -631,7 +658,9 @@ void build_layout(Layout& L, const std::vector<BoxIn>& boxes, const pcg_hydro_pa
   const int qf_grow = (prm->use_hybrid_weno && prm->ppm_type == 1 && prm->weno_scheme == 2) ? 4 : 3;
   L.ns = ns;
   L.esz = single ? 4 : 8;
-  L.march = face_march(boxes);
+  int64_t cells = 0;
+  for (const BoxIn& b : boxes) cells += b.bx.cells();
+  L.march = face_march(cells);
   // the mixed form traces from TMA-staged shared-memory tiles of its FP32 primitive copy
   // (PPM without hybrid WENO, and PLM)
   L.tile_trace = single && !prm->use_hybrid_weno && pcg::trace_tile_species(ns);
@@ -661,7 +690,7 @@ void build_layout(Layout& L, const std::vector<BoxIn>& boxes, const pcg_hydro_pa
     R.zero_uout = B.zero_uout ? 1 : 0;
     const IBox g4 = grow(B.bx, 4), g1 = grow(B.bx, 1);
     // direction segments interleaved in z-slabs for large regions (see add_dir_segs)
-    const bool slabs = ns > 1 && g1.cells() * nv * 8 > kOrderRegionBytes && B.bx.n(2) >= 2 * kOrderSlab;
+    const bool slabs = single && ns > 1 && g1.cells() * nv * 8 > kOrderRegionBytes && B.bx.n(2) >= 2 * kOrderSlab;
     const int z0 = B.bx.lo[2];
     IBox sb[3];
     if (B.internal_q) {
@@ -758,8 +787,8 @@ void build_layout(Layout& L, const std::vector<BoxIn>& boxes, const pcg_hydro_pa
     add_seg(L, K_CONSUP, (int)r, 0, B.bx);
     L.regions.push_back(R);
   }
-  if (boxes.size() > 1)
-    for (int st : {K_FLUX0, K_FLUX1, K_FLUX2}) group_segs(L, st);
+  for (int st : {K_FLUX0, K_FLUX1, K_FLUX2})
+    if (group_by_direction(prm->precision_mode, ns, st, (int64_t)boxes.size(), cells)) group_segs(L, st);
   // alternate traversal directions of successive stages (see add_dir_segs); K_CONSUP
   // keeps one segment per region in region order (the per-box timesteps index it)
   for (int st = K_CTOPRIM; st <= K_FLUX2; ++st)
