@@ -341,13 +341,20 @@ int pcg_average_down(const pcg_array4* fine, pcg_array4* crse, const int32_t fin
 /* Each heavy stage (0 ctoprim, 2 trace, 3-5 Riemann stages) exists in three register
  * budgets (variants 0-2, increasingly tight); the library keeps the variant used
  * per (precision_mode, species class of nspec: 1, 2-5, 6-12 or more, stage). The trace of
- * PCG_PREC_MIXED has variants 3-5 as well: the same budgets for the tiled trace, which stages each tile of the FP32
- * primitive state and its halo in shared memory with one TMA load (plain PPM and PLM;
- * the hybrid-WENO trace is never tiled). particleclem_b200/autotune.py times them and
- * sets the fastest. No counterpart in the reference (AMReX chooses launch shapes). */
+ * PCG_PREC_MIXED has variants 3-5 as well: the same budgets for the tiled trace, which
+ * stages each tile of the FP32 primitive state and its halo in shared memory with one TMA
+ * load (plain PPM and PLM; the hybrid-WENO trace is never tiled).
+ * particleclem_b200/autotune.py times them and sets the fastest. No counterpart in the
+ * reference (AMReX chooses launch shapes).
+ * The library's own choice for 2 to 5 species depends on the size of the launch. A variant
+ * set here holds at every size; setting the one the library reports for large launches
+ * (pcg_get_launch_variant before any other was set) gives the choice back to the library, so
+ * that a variant read and set back changes nothing. */
 int pcg_set_launch_variant(int32_t precision_mode, int32_t nspec, int32_t stage, int32_t variant);
-/* Current variant, or a negative PCG_E* code. */
+/* Current variant of large launches, or a negative PCG_E* code. */
 int pcg_get_launch_variant(int32_t precision_mode, int32_t nspec, int32_t stage);
+/* Variant of a launch of nblocks blocks of 128 threads, or a negative PCG_E* code. */
+int pcg_launch_variant_for(int32_t precision_mode, int32_t nspec, int32_t stage, int64_t nblocks);
 
 #ifdef __cplusplus
 }

@@ -126,13 +126,12 @@ constexpr size_t kAlign = 256;
 thread_local std::string g_err;
 
 // Launch-variant table: [precision_mode][species class][stage] -> variant index of
-// kMinBlocks (pcg_kernels.cuh). Defaults measured on B200 for the production flame
+// kMinBlocks (pcg_kernels.cuh). Measured on B200 for the production flame
 // level; pcg_set_launch_variant (the autotuner) overrides them. The mixed form's trace
 // has three more variants: 3-5 run the TMA-staged tiled trace (K_TRACE_TILE) with the
 // register budgets 0-2.
 constexpr int kTileVariant = 3;
-std::mutex g_var_mu;
-int g_variant[3][4][7] = {
+constexpr int kDefaultVariant[3][4][7] = {
   // one species, 2 to 5 species, 6 to 12, more (whose kernels spill under every cap)
   {{0, 0, 2, 0, 2, 1, 2}, {2, 0, 1, 2, 2, 2, 1}, {2, 0, 2, 1, 0, 0, 2}, {1, 0, 0, 0, 0, 0, 1}},  // FP64 reference order
   {{0, 0, 2, 0, 0, 0, 0}, {2, 0, 1, 2, 2, 2, 1}, {2, 0, 2, 1, 0, 0, 0}, {1, 0, 0, 0, 0, 0, 1}},  // FP64 with FMA
@@ -143,22 +142,27 @@ int g_variant[3][4][7] = {
 // 0.461, with FMA flux1 0.528 -> 0.447, flux2 0.458 -> 0.396, mixed flux1 0.278 -> 0.214. Counts
 // measured: 2 and 3 alike, 9, 21. A launch of one wave (4 blocks per SM, in the FP64 forms, whose
 // tight caps spill more, two such waves) has little to gain from them and takes the next class's
-// caps unless the caller chose the variant. Steps of 3-species levels, us, next class -> tight: 16^3
-// FP64 81.2 -> 83.5, mixed 64.0 -> 64.2; 30^3 FP64 112 -> 120; 34^3 137 -> 143; 36^3 147 -> 144;
+// caps unless the caller chose another variant. Steps of 3-species levels, us, next class -> tight:
+// 16^3 FP64 81.2 -> 83.5, mixed 64.0 -> 64.2; 30^3 FP64 112 -> 120; 34^3 137 -> 143; 36^3 147 -> 144;
 // 48^3 286 -> 260; 33^3 mixed (hybrid WENO) 94.0 -> 86.8.
 enum { FEW_SPECIES = 1 };
+constexpr int kSMs = 148;  // of a B200
 constexpr int kFewBlocksVariant[3][7] = {{2, 0, 2, 1, 1, 0, 2}, {2, 0, 2, 1, 0, 0, 0}, {2, 0, 0, 0, 1, 1, 2}};
-constexpr int64_t kFewBlocks[3] = {8 * 148, 8 * 148, 4 * 148};
-bool g_chosen[3][4][7];
+constexpr int64_t kFewBlocks[3] = {8 * kSMs, 8 * kSMs, 4 * kSMs};
+// The caller's choices, variant + 1. Choosing the table's own variant is choosing the library's
+// rule again, so that a variant read and set back (or saved and restored around a tuning) leaves
+// the library as it was.
+std::mutex g_var_mu;
+int g_choice[3][4][7];
 int species_class(int ns) { return ns == 1 ? 0 : ns <= 5 ? FEW_SPECIES : ns <= 12 ? 2 : 3; }
 int max_variant(int prec, int stage) { return (prec == PCG_PREC_MIXED && stage == K_TRACE) ? 5 : 2; }
 // The variant of a launch of nblocks blocks.
 int variant_of(int prec, int ns, int stage, int64_t nblocks) {
   std::lock_guard<std::mutex> lk(g_var_mu);
-  const int cls = species_class(ns);
-  if (cls == FEW_SPECIES && nblocks <= kFewBlocks[prec] && !g_chosen[prec][cls][stage])
-    return kFewBlocksVariant[prec][stage];
-  return g_variant[prec][cls][stage];
+  const int cls = species_class(ns), chosen = g_choice[prec][cls][stage];
+  if (chosen) return chosen - 1;
+  if (cls == FEW_SPECIES && nblocks <= kFewBlocks[prec]) return kFewBlocksVariant[prec][stage];
+  return kDefaultVariant[prec][cls][stage];
 }
 
 // Stream-ordered workspace pool per device. Its release threshold is unbounded, so
@@ -1979,15 +1983,19 @@ int pcg_set_launch_variant(int32_t precision_mode, int32_t nspec, int32_t stage,
       variant < 0 || variant > max_variant(precision_mode, stage))
     return fail(PCG_EINVAL, "launch variant (%d, %d, %d, %d) out of range", precision_mode, nspec, stage, variant);
   std::lock_guard<std::mutex> lk(g_var_mu);
-  g_variant[precision_mode][species_class(nspec)][stage] = variant;
-  g_chosen[precision_mode][species_class(nspec)][stage] = true;
+  const int cls = species_class(nspec);
+  g_choice[precision_mode][cls][stage] = variant == kDefaultVariant[precision_mode][cls][stage] ? 0 : variant + 1;
   return PCG_OK;
 }
 
 int pcg_get_launch_variant(int32_t precision_mode, int32_t nspec, int32_t stage) {
-  if (precision_mode < 0 || precision_mode > 2 || !species_built(nspec) || stage < 0 || stage >= K_NSTAGE)
+  return pcg_launch_variant_for(precision_mode, nspec, stage, INT64_MAX);
+}
+
+int pcg_launch_variant_for(int32_t precision_mode, int32_t nspec, int32_t stage, int64_t nblocks) {
+  if (precision_mode < 0 || precision_mode > 2 || !species_built(nspec) || stage < 0 || stage >= K_NSTAGE || nblocks < 0)
     return fail(PCG_EINVAL, "launch variant query out of range");
-  return variant_of(precision_mode, nspec, stage, INT64_MAX);
+  return variant_of(precision_mode, nspec, stage, nblocks);
 }
 
 int pcg_plan_destroy(pcg_plan* P) {

@@ -87,6 +87,7 @@ SIGNATURES = {
     "pcg_plan_destroy": ([_V], C.c_int),
     "pcg_set_launch_variant": ([C.c_int32, C.c_int32, C.c_int32, C.c_int32], C.c_int),
     "pcg_get_launch_variant": ([C.c_int32, C.c_int32, C.c_int32], C.c_int),
+    "pcg_launch_variant_for": ([C.c_int32, C.c_int32, C.c_int32, C.c_int64], C.c_int),
 }
 
 _lib = None

@@ -1,10 +1,11 @@
 """GPU tests that the launch rules change no result: the order of the stage segments in calls
-of many regions, on both sides of the sizes where it changes."""
+of many regions and the register caps of few species, on both sides of the sizes where they
+change."""
 import numpy as np
 import pytest
 
 from common import eos9, gpu_zeros, oracle, params_for, to_cpu, to_gpu
-from particleclem_b200 import abi, hydro, workloads as wl
+from particleclem_b200 import abi, hydro, native, thermo, workloads as wl
 
 pytestmark = pytest.mark.gpu
 FORMS = [abi.PREC_FP64, abi.PREC_FP64_FAST, abi.PREC_MIXED]
@@ -35,3 +36,29 @@ def test_boxes_of_one_call_equal_calls_of_one_box(prec, nspec, edges, count):
         a = to_cpu(a)
         assert np.isfinite(a).all()
         np.testing.assert_array_equal(a, to_cpu(b))
+
+
+@pytest.mark.parametrize("nspec", [2, 3])
+@pytest.mark.parametrize("edges", [(35, 34, 33), (52, 47, 45)])
+def test_few_species_equal_oracle_where_every_stage_changes_its_caps(nspec, edges):
+    """The second Riemann stage, whose marches of two y- or z-faces per thread make the fewest
+    blocks, launches 1755 blocks of the larger box (876 + 439 + 440)."""
+    if nspec not in hydro.species_counts():
+        pytest.skip(f"library built without {nspec} species")
+    nx, ny, nz = edges
+    cells, march = nx * ny * nz, 1 if nx * ny * nz <= 60000 else 2
+    threads = ((nx + 1) * ny * nz, nx * nz * -(-(ny + 1) // march), nx * ny * -(-(nz + 1) // march))
+    blocks = sum(-(-t // 128) for t in threads)
+    assert cells <= 120000 and (blocks > 1184) == (edges[0] == 52)
+    lib = native.load()
+    assert lib.pcg_launch_variant_for(abi.PREC_FP64, nspec, 5, blocks) == (2 if blocks > 1184 else 0)
+    eos = thermo.standin_mixture(nspec)
+    hydro.init(0)
+    hydro.set_eos(eos)
+    oracle().set_eos(eos)
+    p = wl.random_patch(edges, 18, eos)
+    prm = params_for(p, 0.3 * oracle().estdt(p.lo, p.hi, p.fab, p.dx), prec=abi.PREC_FP64, nspec=nspec)
+    ref, _ = oracle().hydro_box(prm, p.lo, p.hi, p.fab)
+    out = gpu_zeros(abi.nvar(nspec), p.lo, p.hi)
+    hydro.hydro_box(prm, p.lo, p.hi, to_gpu(p.fab), out)
+    np.testing.assert_array_equal(to_cpu(out), ref.data)
