@@ -1862,10 +1862,11 @@ __device__ __forceinline__ void consup_each(const pcg::Region& rg, int i, int j,
   constexpr int NV = pcg::nvar(NS);
   const FinalView<F, NV> f0(rg.ff[0], 0, i, j, k), f1(rg.ff[1], 1, i, j, k), f2(rg.ff[2], 2, i, j, k);
   const double v = rg.vol.p ? v4<const double>(rg.vol)(i, j, k) : rg.vol_u;
-  const auto pdivu_sum = [&] {
+  // the faces' pressures and velocities, low and high, and areas (loaded ahead of the fluxes)
+  double q0[2], q0p[2], q1[2], q1p[2], q2[2], q2p[2], a0m, a0p, a1m, a1p, a2m, a2p;
+  if constexpr (EINT) {
     const FinalView<F, 2> e0(rg.qec[0], 0, i, j, k), e1(rg.qec[1], 1, i, j, k), e2(rg.qec[2], 2, i, j, k);
     constexpr int VE = FinalView<F, 2>::V;
-    double q0[2], q0p[2], q1[2], q1p[2], q2[2], q2p[2];
 #pragma unroll
     for (int n0 = 0; n0 < 2; n0 += VE) {
       e0.get(n0, q0 + n0, q0p + n0);
@@ -1876,9 +1877,11 @@ __device__ __forceinline__ void consup_each(const pcg::Region& rg, int i, int j,
     const V4<const double> a0 = v4<const double>(rg.area[0]);
     const V4<const double> a1 = v4<const double>(rg.area[1]);
     const V4<const double> a2 = v4<const double>(rg.area[2]);
-    const double a0m = ua ? a0(i, j, k) : rg.area_u[0], a0p = ua ? a0(i + 1, j, k) : rg.area_u[0];
-    const double a1m = ua ? a1(i, j, k) : rg.area_u[1], a1p = ua ? a1(i, j + 1, k) : rg.area_u[1];
-    const double a2m = ua ? a2(i, j, k) : rg.area_u[2], a2p = ua ? a2(i, j, k + 1) : rg.area_u[2];
+    a0m = ua ? a0(i, j, k) : rg.area_u[0], a0p = ua ? a0(i + 1, j, k) : rg.area_u[0];
+    a1m = ua ? a1(i, j, k) : rg.area_u[1], a1p = ua ? a1(i, j + 1, k) : rg.area_u[1];
+    a2m = ua ? a2(i, j, k) : rg.area_u[2], a2p = ua ? a2(i, j, k + 1) : rg.area_u[2];
+  }
+  const auto pdivu_sum = [&] {
     return 0.5 * ((q0p[0] + p0 + (q0[0] + p0)) * (q0p[1] * a0p - q0[1] * a0m) +
                   (q1p[0] + p0 + (q1[0] + p0)) * (q1p[1] * a1p - q1[1] * a1m) +
                   (q2p[0] + p0 + (q2[0] + p0)) * (q2p[1] * a2p - q2[1] * a2m));
