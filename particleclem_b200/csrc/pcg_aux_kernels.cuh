@@ -117,12 +117,9 @@ __global__ void __launch_bounds__(kFinalThreads) k_estdt_final(const __grid_cons
   cl.sync();  // the minima stay readable until block 0 is done
 }
 
-// Source/Advance.cpp:397-417 (construct_Snew, hydro only) then Source/PeleC.cpp:2289-2305
-// (computeTemp): pc_rst_int_e default branch (PeleCUtilities.H:227-235) and pc_cmpTemp
-// (PeleCUtilities.H:70-84), on one cell: s holds S_old on entry and S_new on exit.
-// construct_Snew's pc_rst_int_e and computeTemp on the state s (already S_old + dt *
-// hydro source).
-// The internal energy of S_new into s (pc_rst_int_e), its mass fractions into y; returns e.
+// The energy step of pc_rst_int_e (default branch, PeleCUtilities.H:227-235) on a state s that
+// already holds S_old + dt * hydro source: the internal energy into s, the mass fractions into
+// y; returns the specific internal energy.
 template <int NS>
 __device__ __forceinline__ double energy_cell(double* s, double* y) {
   const double rho = s[pcg::URHO];
@@ -138,6 +135,7 @@ __device__ __forceinline__ double energy_cell(double* s, double* y) {
   for (int n = 0; n < NS; ++n) y[n] = s[pcg::UFS + n] * rhoInv2;
   return e;
 }
+// pc_rst_int_e and computeTemp (pc_cmpTemp, PeleCUtilities.H:70-84) on such a state.
 template <int NS, bool MIX>
 __device__ __forceinline__ void finish_cell(double* s) {
   using E = Eos<NS, MIX, double>;
@@ -145,7 +143,10 @@ __device__ __forceinline__ void finish_cell(double* s) {
   const double e = energy_cell<NS>(s, y);
   s[pcg::UTEMP] = E::rey2t(e, y, s[pcg::UTEMP]);
 }
-// finish_cell and the CFL constraint of the result in one, sharing the mixture polynomial.
+// finish_cell and the CFL constraint of the result. With one range switch temperature the
+// reduced forms solve for T on the mixture polynomial and take the sound speed from it: the
+// values of finish_cell and cfl_dt but for FP64 rounding. The reference-order form and tables with
+// several switch temperatures call the two.
 template <int NS, bool MIX>
 __device__ __forceinline__ double finish_cfl(double* s, const double* dx) {
   if (MIX && !kExact && EosC<double, MIX>::uniform_tmid()) {
@@ -162,6 +163,8 @@ __device__ __forceinline__ double finish_cfl(double* s, const double* dx) {
   return cfl_dt<NS, MIX>(s, dx);
 }
 
+// Source/Advance.cpp:397-417 (construct_Snew, hydro only) then Source/PeleC.cpp:2289-2305
+// (computeTemp) on one cell: s holds S_old on entry and S_new on exit.
 template <int NS, bool MIX>
 __device__ __forceinline__ void update_cell(double* s, const double* hsrc, double dt) {
 #pragma unroll
@@ -194,8 +197,9 @@ __global__ void __launch_bounds__(128) k_update(const __grid_constant__ pcg::Aux
 // written), S_new = S_old + dt * hydro_source with computeTemp written over the state in
 // place, and the CFL constraint of S_new for the next step (block minima; the final
 // minimum is k_estdt_final). In place: a thread reads and writes the state of its own cell
-// only. Each value is formed by the same expressions as k_consup,
-// k_update and k_estdt, so the step is the unfused step's.
+// only. The step is the unfused one's (k_consup, k_update, k_estdt): bit for bit in the
+// reference-order form; in the reduced forms temperature and timestep differ by FP64 rounding
+// (finish_cfl).
 template <int NS, bool MIX, int MINB>
 __global__ void __launch_bounds__(128, MINB) k_advance(const __grid_constant__ pcg::StageArgs a) {
   Item it;

@@ -122,11 +122,6 @@ __device__ __forceinline__ double div_one(double x, double b, double r, bool bok
   const int sign = (__double2hiint(x) ^ __double2hiint(b)) & 0x80000000;
   return __hiloint2double((__double2hiint(q2) & 0x7fffffff) | sign, __double2loint(q2));
 }
-template <int N>
-__device__ __forceinline__ void div_all(const float* x, float b, float* q) {
-#pragma unroll
-  for (int n = 0; n < N; ++n) q[n] = x[n] / b;
-}
 
 // ------------------------------------------------------------------ views
 // Element offsets within one view are 32-bit: the host refuses arrays whose component
@@ -405,7 +400,6 @@ struct Eos {
     }
     return tt;
   }
-  static __device__ __forceinline__ R rty2p(R r, R t, const R* y) { return r * rmix(y) * t; }
   static __device__ __forceinline__ R rty2cs(R r, R t, const R* y) {
     const R rm = rmix(y);
     const R p = r * rm * t;
@@ -414,22 +408,9 @@ struct Eos {
     const R g = (cv + rm) / cv;
     return sqrt(g * p / r);
   }
-  static __device__ __forceinline__ R rty2g(R t, const R* y) {
-    if (!MIX) return C::gamma();
-    const R cv = cv_of(t, y);
-    return (cv + rmix(y)) / cv;
-  }
-  static __device__ __forceinline__ void rty2dpde_dpdre(R r, R t, const R* y, R& dpde, R& dpdr_e) {
-    const R rm = rmix(y);
-    if (!MIX) {
-      dpde = (C::gamma() - R(1)) * r;
-    } else {
-      dpde = r * rm / cv_of(t, y);
-    }
-    dpdr_e = rm * t;
-  }
   // RTY2P, RTY2Cs and RTY2G of one state, sharing rmix and cv (left in rm, cv for
-  // dpde_dpdre): each value is formed by exactly the operations of the separate calls.
+  // dpde_dpdre, which is RTY2dpde_dpdre): each value is formed by exactly the operations of
+  // the separate calls.
   static __device__ __forceinline__ void rty2pcg(R r, R t, const R* y, R& p, R& cs, R& g, R& rm, R& cv) {
     rm = rmix(y);
     p = r * rm * t;
@@ -1114,7 +1095,7 @@ __device__ __forceinline__ void cmpflx(const R* ql, const R* qr, int idx, int bc
     }
   }
   RiemannOut<R> o;
-  if (EXACT)
+  if constexpr (EXACT)
     riemann<NS, MIX, R>(L, Rs, cav, o);
   else
     riemann_reduced<NS, MIX, R>(L, Rs, cav, p0, o);

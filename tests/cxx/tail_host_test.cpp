@@ -5,6 +5,10 @@
 //                          first row, whose state lies on pages that cannot be read: a tail
 //                          that reads another cell's state, which its own thread may be
 //                          replacing meanwhile, ends with SIGSEGV
+//   tail_host_test energy FILE   FILE: an EOS table (mw, switch temperatures, low and high
+//                          coefficients of 9 species), int32 n, n states [e, T guess, Y]; prints
+//                          per state T of the fused tail and of the update, then the CFL bound of
+//                          the fused tail and of estdt
 #include <cuda_runtime.h>
 #include <sys/mman.h>
 
@@ -153,6 +157,53 @@ int run_cells() {
   return 0;
 }
 
+int run_energy(const char* path) {
+  FILE* f = std::fopen(path, "rb");
+  if (!f) return 1;
+  pcg::EosConst& c = c_eos[1];
+  c = pcg::EosConst{};
+  c.kind = 1;
+  c.nspec = NS;
+  double mw[NS], tmid[NS], al[2][NS][7];
+  size_t got = std::fread(mw, 8, NS, f) + std::fread(tmid, 8, NS, f) + std::fread(al, 8, 2 * NS * 7, f);
+  int32_t n = 0;
+  got += std::fread(&n, 4, 1, f);
+  if (got != size_t(2 * NS + 14 * NS + 1)) return 1;
+  c.uniform_tmid = 1;
+  for (int k = 0; k < NS; ++k) {
+    const double rw = pcg::RU / mw[k];
+    c.imw[k] = 1.0 / mw[k];
+    c.tmid[k] = tmid[k];
+    if (tmid[k] != tmid[0]) c.uniform_tmid = 0;
+    for (int r = 0; r < 2; ++r) {
+      const double* a = al[r][k];
+      for (int i = 0; i < 5; ++i) c.cvc[k][r][i] = rw * (a[i] - (i == 0));
+      c.ec[k][r][0] = rw * a[5];
+      for (int i = 0; i < 5; ++i) c.ec[k][r][i + 1] = rw * ((a[i] - (i == 0)) / (i + 1));
+    }
+  }
+  const double dx[3] = {1.0, 1.5, 2.0};
+  for (int m = 0; m < n; ++m) {
+    double in[2 + NS], s[2][NV];
+    if (std::fread(in, 8, 2 + NS, f) != size_t(2 + NS)) return 1;
+    const double rho = 1.3e-3, v[3] = {2e3, -1e3, 5e2};
+    for (auto& q : s) {
+      q[pcg::URHO] = rho;
+      double ke = 0.0;
+      for (int d = 0; d < 3; ++d) q[pcg::UMX + d] = rho * v[d], ke += 0.5 * v[d] * v[d];
+      q[pcg::UEDEN] = rho * (in[0] + ke);
+      q[pcg::UEINT] = 0.0;
+      q[pcg::UTEMP] = in[1];
+      for (int k = 0; k < NS; ++k) q[pcg::UFS + k] = rho * in[2 + k];
+    }
+    const double fused = finish_cfl<NS, true>(s[0], dx);
+    finish_cell<NS, true>(s[1]);
+    std::printf("%.17g %.17g %.17g %.17g\n", s[0][pcg::UTEMP], s[1][pcg::UTEMP], fused, cfl_dt<NS, true>(s[1], dx));
+  }
+  std::fclose(f);
+  return 0;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -161,5 +212,6 @@ int main(int argc, char** argv) {
     const int a = run_cells<float>();
     return a ? a : run_cells<double>();
   }
+  if (argc == 3 && !std::strcmp(argv[1], "energy")) return run_energy(argv[2]);
   return 64;
 }
