@@ -580,11 +580,12 @@ void group_segs(Layout& L, int stage) {
   }
 }
 
-// Which of the two orders a call of many regions takes, by the size of its regions (mean
-// cells). The large kernels (FP64 in reference order, and with FMA from 6 species) always gain
-// from whole directions; the smaller ones only while a region's direction is too few blocks
-// to fill the chip, flux1 up to larger regions than flux0 and flux2; with one species only in
-// calls of a few waves. ms, region order / by direction, flux0, flux1, flux2:
+// Which of the two orders a call of many regions takes, by the size of the regions most of its
+// cells are in (region_cells: their mean, weighted by cells). The large kernels (FP64 in
+// reference order, and with FMA from 6 species) always gain from whole directions; the smaller
+// ones only while a region's direction is too few blocks to fill the chip, flux1 up to larger
+// regions than flux0 and flux2; with one species only in calls of a few waves. ms, region order /
+// by direction, flux0, flux1, flux2 (a - b: edges log-uniform in that range):
 //   9 species FP64   64 x 32^3  1.03 / .940   3.21 / 2.91   2.03 / 1.92
 //                     8 x 64^3  .978 / .854   2.73 / 2.68   1.99 / 1.84
 //   9 species mixed 300 x 12^3  .146 / .130   .403 / .334   .283 / .256
@@ -592,20 +593,25 @@ void group_segs(Layout& L, int stage) {
 //                    40 x 28^3  .158 / .156   .440 / .404   .336 / .342
 //                    64 x 32^3  .344 / .347   .933 / .881   .702 / .762
 //                     6 x 56^3  .143 / .157   .418 / .420   .342 / .363
+//                200 x 8 - 32   .236 / .210   .638 / .544   .465 / .448
+//                200 x 8 - 64   .607 / .573   1.71 / 1.54   1.28 / 1.31
 //   3 species mixed  24 x 32^3  .090 / .088   .223 / .207   .197 / .203
 //                     6 x 64^3  .133 / .137   .339 / .342   .334 / .360
+//                200 x 8 - 64   .386 / .374   .973 / .890   .876 / .916
 //   2 species FMA    16 x 40^3  .151 / .150   .436 / .410   .344 / .356
 //   one species FP64 32 x 16^3  .027 / .027   .060 / .057   .061 / .051
 //                    64 x 32^3  .253 / .264   .632 / .650   .576 / .611
 //   one species mixed 8 x 32^3  .023 / .023   .057 / .053   .055 / .051
 //                    64 x 32^3  .143 / .150   .352 / .378   .329 / .375
-constexpr int64_t kGroupCells = 20000, kGroupCellsFlux1 = 200000;
-constexpr int64_t kGroupCellsOne = 40000, kGroupCallCellsOne = int64_t(1) << 18;
-bool group_by_direction(int prec, int ns, int stage, int64_t regions, int64_t cells) {
+//                200 x 8 - 64   .245 / .255   .591 / .640   .562 / .647
+constexpr double kGroupCells[3] = {40000, 200000, 20000};  // flux0, flux1, flux2
+constexpr double kGroupCellsOne = 40000;
+constexpr int64_t kGroupCallCellsOne = int64_t(1) << 18;
+bool group_by_direction(int prec, int ns, int stage, size_t regions, double region_cells, int64_t cells) {
   if (regions < 2) return false;
-  if (ns == 1) return cells / regions <= kGroupCellsOne && cells <= kGroupCallCellsOne;
+  if (ns == 1) return region_cells <= kGroupCellsOne && cells <= kGroupCallCellsOne;
   if (prec == PCG_PREC_FP64 || (prec == PCG_PREC_FP64_FAST && ns > 5)) return true;
-  return cells / regions <= (stage == K_FLUX1 ? kGroupCellsFlux1 : kGroupCells);
+  return region_cells <= kGroupCells[stage - K_FLUX0];
 }
 
 // The tiled trace of direction d over g1 = grow(box,1), as K_TRACE_TILE segments: the up
@@ -663,7 +669,12 @@ void build_layout(Layout& L, const std::vector<BoxIn>& boxes, const pcg_hydro_pa
   L.ns = ns;
   L.esz = single ? 4 : 8;
   int64_t cells = 0;
-  for (const BoxIn& b : boxes) cells += b.bx.cells();
+  double region_cells = 0.0;
+  for (const BoxIn& b : boxes) {
+    cells += b.bx.cells();
+    region_cells += double(b.bx.cells()) * b.bx.cells();
+  }
+  region_cells /= cells;
   L.march = face_march(cells);
   // the mixed form traces from TMA-staged shared-memory tiles of its FP32 primitive copy
   // (PPM without hybrid WENO, and PLM)
@@ -792,7 +803,7 @@ void build_layout(Layout& L, const std::vector<BoxIn>& boxes, const pcg_hydro_pa
     L.regions.push_back(R);
   }
   for (int st : {K_FLUX0, K_FLUX1, K_FLUX2})
-    if (group_by_direction(prm->precision_mode, ns, st, (int64_t)boxes.size(), cells)) group_segs(L, st);
+    if (group_by_direction(prm->precision_mode, ns, st, boxes.size(), region_cells, cells)) group_segs(L, st);
   // alternate traversal directions of successive stages (see add_dir_segs); K_CONSUP
   // keeps one segment per region in region order (the per-box timesteps index it)
   for (int st = K_CTOPRIM; st <= K_FLUX2; ++st)

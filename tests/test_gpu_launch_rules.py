@@ -14,10 +14,11 @@ FORMS = [abi.PREC_FP64, abi.PREC_FP64_FAST, abi.PREC_MIXED]
 @pytest.mark.parametrize("prec", FORMS)
 @pytest.mark.parametrize("nspec,edges,count", [
     (1, (7, 5, 6), 3), (1, (35, 34, 33), 6), (1, (35, 34, 33), 7), (1, (35, 35, 34), 2),
-    (9, (7, 5, 6), 5), (9, (27, 28, 26), 2), (9, (27, 28, 27), 2), (9, (59, 58, 58), 2), (9, (59, 59, 58), 2)])
+    (9, (7, 5, 6), 5), (9, (27, 28, 26), 2), (9, (27, 28, 27), 2), (9, (35, 34, 33), 2), (9, (35, 35, 34), 2),
+    (9, (59, 58, 58), 2), (9, (59, 59, 58), 2)])
 def test_boxes_of_one_call_equal_calls_of_one_box(prec, nspec, edges, count):
-    """Around 40000 cells per region and 2^18 per call with one species, 20000 and 200000
-    per region for mixtures."""
+    """Around 40000 cells per region and 2^18 per call with one species, 20000, 40000 and
+    200000 per region for mixtures."""
     eos = wl.GammaLaw() if nspec == 1 else eos9()
     hydro.init(0)
     hydro.set_eos(eos)
