@@ -676,6 +676,9 @@ void build_layout(Layout& L, const std::vector<BoxIn>& boxes, const pcg_hydro_pa
   }
   region_cells /= cells;
   L.march = face_march(cells);
+  const auto grouped = [&](int stage) {
+    return group_by_direction(prm->precision_mode, ns, stage, boxes.size(), region_cells, cells);
+  };
   // the mixed form traces from TMA-staged shared-memory tiles of its FP32 primitive copy
   // (PPM without hybrid WENO, and PLM)
   L.tile_trace = single && !prm->use_hybrid_weno && pcg::trace_tile_species(ns);
@@ -704,8 +707,10 @@ void build_layout(Layout& L, const std::vector<BoxIn>& boxes, const pcg_hydro_pa
     for (int d = 0; d < 3; ++d) R.area[d] = B.area[d];
     R.zero_uout = B.zero_uout ? 1 : 0;
     const IBox g4 = grow(B.bx, 4), g1 = grow(B.bx, 1);
-    // direction segments interleaved in z-slabs for large regions (see add_dir_segs)
-    const bool slabs = single && ns > 1 && g1.cells() * nv * 8 > kOrderRegionBytes && B.bx.n(2) >= 2 * kOrderSlab;
+    // k_flux2's direction segments interleaved in z-slabs for large regions (see add_dir_segs),
+    // unless group_segs is to sort them by direction
+    const bool slabs = single && ns > 1 && !grouped(K_FLUX2) && g1.cells() * nv * 8 > kOrderRegionBytes &&
+                       B.bx.n(2) >= 2 * kOrderSlab;
     const int z0 = B.bx.lo[2];
     IBox sb[3];
     if (B.internal_q) {
@@ -803,7 +808,7 @@ void build_layout(Layout& L, const std::vector<BoxIn>& boxes, const pcg_hydro_pa
     L.regions.push_back(R);
   }
   for (int st : {K_FLUX0, K_FLUX1, K_FLUX2})
-    if (group_by_direction(prm->precision_mode, ns, st, boxes.size(), region_cells, cells)) group_segs(L, st);
+    if (grouped(st)) group_segs(L, st);
   // alternate traversal directions of successive stages (see add_dir_segs); K_CONSUP
   // keeps one segment per region in region order (the per-box timesteps index it)
   for (int st = K_CTOPRIM; st <= K_FLUX2; ++st)
