@@ -63,3 +63,42 @@ def test_few_species_equal_oracle_where_every_stage_changes_its_caps(nspec, edge
     out = gpu_zeros(abi.nvar(nspec), p.lo, p.hi)
     hydro.hydro_box(prm, p.lo, p.hi, to_gpu(p.fab), out)
     np.testing.assert_array_equal(to_cpu(out), ref.data)
+
+
+@pytest.mark.parametrize("prec", FORMS)
+def test_steps_overlapping_on_two_streams_equal_steps_waited_for(prec):
+    """Patches stepped on two streams at once, each call's launches overlapping, against the
+    same steps with a wait after each."""
+    import torch
+
+    eos = eos9()
+    hydro.init(0)
+    hydro.set_eos(eos)
+    sets = [[wl.flame_patch(e, 60 + k, eos) for k, e in enumerate(edges)]
+            for edges in ([(8, 12, 6), (12, 9, 11)], [(16, 8, 8), (5, 7, 11), (9, 10, 12)])]
+    prm = abi.make_params((1, 1, 1), 0.0, 9, (0, 0, 0), (0, 0, 0), (0, 0, 0), (0, 0, 0), precision_mode=prec)
+    bc = (abi.BC_OUTFLOW,) * 3
+
+    def start(patches):
+        states = [to_gpu(p.fab) for p in patches]
+        boxes = [hydro.make_box(p.lo, p.hi, s, None, p.dx, 0.0, p.lo, p.hi, bc, bc) for p, s in zip(patches, states)]
+        dt = torch.full((len(patches),), 1e-9, dtype=torch.float64, device="cuda")
+        return states, boxes, dt, torch.empty_like(dt)
+
+    results = []
+    for wait in (True, False):
+        runs = [start(p) for p in sets]
+        streams = [torch.cuda.Stream() for _ in sets]
+        torch.cuda.synchronize()
+        for _ in range(6):
+            for m, (_, boxes, dt, dt_next) in enumerate(runs):
+                # no copies on the streams: successive steps swap the two timestep arrays
+                hydro.step_boxes(prm, boxes, 0.3, dt, dt_next, stream=streams[m])
+                runs[m] = (runs[m][0], boxes, dt_next, dt)
+                if wait:
+                    torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        results.append([to_cpu(s) for r in runs for s in r[0]] + [r[2].cpu().numpy() for r in runs])
+    for a, b in zip(*results):
+        assert np.isfinite(a).all()
+        np.testing.assert_array_equal(a, b)
